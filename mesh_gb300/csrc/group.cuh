@@ -47,6 +47,13 @@ template <class T> MESH_HD cx<T> csub(cx<T> a, cx<T> b) { return {a.re - b.re, a
 template <class T> MESH_HD cx<T> cconj(cx<T> a) { return {a.re, -a.im}; }
 template <class T> MESH_HD cx<T> cscale(cx<T> a, T s) { return {a.re * s, a.im * s}; }
 
+// a x + b y: each real part one multiply and three fused multiply-adds
+template <class T> MESH_HD cx<T> cmul2(cx<T> a, cx<T> x, cx<T> b, cx<T> y)
+{
+	return {fma(a.re, x.re, fma(-a.im, x.im, fma(b.re, y.re, -b.im * y.im))),
+	        fma(a.re, x.im, fma(a.im, x.re, fma(b.re, y.im, b.im * y.re)))};
+}
+
 template <class T> MESH_HD T m_sqrt(T x) { return sqrt(x); }
 template <class T> MESH_HD T m_rsqrt(T x) { return T(1) / sqrt(x); }
 template <class T> MESH_HD void m_sincos(T x, T *s, T *c)
@@ -57,6 +64,7 @@ template <class T> MESH_HD void m_sincos(T x, T *s, T *c)
 #ifdef __CUDA_ARCH__
 template <> __device__ __forceinline__ void m_sincos<float>(float x, float *s, float *c) { sincosf(x, s, c); }
 template <> __device__ __forceinline__ void m_sincos<double>(double x, double *s, double *c) { sincos(x, s, c); }
+template <> __device__ __forceinline__ double m_rsqrt<double>(double x) { return rsqrt(x); }
 #endif
 
 enum
@@ -278,10 +286,63 @@ template <class T> struct Group<SU3, T>
 		r.v[0] = r.v[8] = r.v[16] = T(1);
 		return r;
 	}
+	// Products of FP64 matrices are chains of fused multiply-adds: each real
+	// part one multiply and five fused multiply-adds (108 FP64 operations a
+	// product), where sums of a.re b.re - a.im b.im pairs compile to a
+	// multiply, a fused multiply-add and an add (144 to 162). GB300 issues an
+	// FP64 operation at a small fraction of the FP32 rate, so every FP64 kernel
+	// of SU(3) is bound by their number. FP32 products keep the pairs: their
+	// hot users have packed forms (Su3F2), and the heat-bath's accept tests
+	// compare draws with what these roundings give.
+	static constexpr bool kChain = sizeof(T) == 8;
+	// r (ADD: += ) sum_k A(i, k) B(k, j) for the rows i < NRW
+	template <int NRW, bool ADD, class FA, class FB> MESH_HD static void chain(E &r, FA A, FB B)
+	{
+#pragma unroll
+		for (int i = 0; i < NRW; ++i)
+#pragma unroll
+			for (int j = 0; j < 3; ++j)
+			{
+				cx<T> x = A(i, 0), y = B(0, j);
+				T re = ADD ? fma(x.re, y.re, r.v[6 * i + 2 * j]) : x.re * y.re;
+				T im = ADD ? fma(x.re, y.im, r.v[6 * i + 2 * j + 1]) : x.re * y.im;
+				re = fma(-x.im, y.im, re);
+				im = fma(x.im, y.re, im);
+#pragma unroll
+				for (int k = 1; k < 3; ++k)
+				{
+					x = A(i, k), y = B(k, j);
+					re = fma(x.re, y.re, re);
+					im = fma(x.re, y.im, im);
+					re = fma(-x.im, y.im, re);
+					im = fma(x.im, y.re, im);
+				}
+				r.v[6 * i + 2 * j] = re;
+				r.v[6 * i + 2 * j + 1] = im;
+			}
+	}
+	// s += a b^dagger;  s += a^dagger b;  s += (a b)^dagger, the sums inside the chains
+	MESH_HD static void add_nd(E &s, E const &a, E const &b)
+	{
+		chain<3, true>(s, [&](int i, int k) { return a.at(i, k); }, [&](int k, int j) { return cconj(b.at(j, k)); });
+	}
+	MESH_HD static void add_dn(E &s, E const &a, E const &b)
+	{
+		chain<3, true>(s, [&](int i, int k) { return cconj(a.at(k, i)); }, [&](int k, int j) { return b.at(k, j); });
+	}
+	MESH_HD static void add_mul_adj(E &s, E const &a, E const &b)
+	{
+		chain<3, true>(s, [&](int i, int k) { return cconj(b.at(k, i)); }, [&](int k, int j) { return cconj(a.at(j, k)); });
+	}
 	// c = a * b
 	MESH_HD static E mul(E const &a, E const &b)
 	{
 		E r;
+		if constexpr (kChain)
+		{
+			chain<3, false>(r, [&](int i, int k) { return a.at(i, k); }, [&](int k, int j) { return b.at(k, j); });
+			return r;
+		}
 #pragma unroll
 		for (int i = 0; i < 3; ++i)
 #pragma unroll
@@ -305,6 +366,12 @@ template <class T> struct Group<SU3, T>
 	MESH_HD static E mul_r2(E const &a, E const &b)
 	{
 		E r;
+		if constexpr (kChain)
+		{
+			chain<2, false>(r, [&](int i, int k) { return a.at(i, k); }, [&](int k, int j) { return b.at(k, j); });
+			complete_row2(r);
+			return r;
+		}
 #pragma unroll
 		for (int i = 0; i < 2; ++i)
 #pragma unroll
@@ -327,6 +394,11 @@ template <class T> struct Group<SU3, T>
 	MESH_HD static E mul_nd(E const &a, E const &b)
 	{
 		E r;
+		if constexpr (kChain)
+		{
+			chain<3, false>(r, [&](int i, int k) { return a.at(i, k); }, [&](int k, int j) { return cconj(b.at(j, k)); });
+			return r;
+		}
 #pragma unroll
 		for (int i = 0; i < 3; ++i)
 #pragma unroll
@@ -350,6 +422,11 @@ template <class T> struct Group<SU3, T>
 	MESH_HD static E mul_dn(E const &a, E const &b)
 	{
 		E r;
+		if constexpr (kChain)
+		{
+			chain<3, false>(r, [&](int i, int k) { return cconj(a.at(k, i)); }, [&](int k, int j) { return b.at(k, j); });
+			return r;
+		}
 #pragma unroll
 		for (int i = 0; i < 3; ++i)
 #pragma unroll
@@ -484,7 +561,7 @@ template <class T> struct Group<SU3, T>
 	}
 	// exp(X) for antihermitian traceless X with |X| < 1 (Frobenius norm), as
 	// the power series truncated after X^N (N = 10: remainder below
-	// |X|^11/11! = 2.5e-8; N = 6 for |X| < 0.2: below 0.2^7/7! = 2.5e-9) and
+	// |X|^11/11! = 2.5e-8; N = 6 for |X| < 0.2: below 0.2^7/7! = 2.5e-9; FP64: N = 18 and 11) and
 	// reduced to a polynomial u0 + u1 X + u2 X^2 with the Cayley-Hamilton
 	// relation X^3 = -c1 X + i dim, c1 = |X|^2/2, i dim = det X; the series
 	// is summed by Horner's rule on the three coefficients (M. Luscher,
@@ -492,9 +569,9 @@ template <class T> struct Group<SU3, T>
 	// the FP32 trajectory's link update.
 	template <int N = 10> MESH_HD static E exp_series(E const &X, E const &X2, T c1, T dim)
 	{
-		static_assert(N >= 1 && N <= 10, "series order");
+		static_assert(N >= 1 && N <= 18, "series order");
 		// 1/k! for k = 0..N
-		constexpr T inv_fact[11] = {T(1),
+		constexpr T inv_fact[19] = {T(1),
 		                               T(1),
 		                               T(1.0 / 2),
 		                               T(1.0 / 6),
@@ -504,7 +581,15 @@ template <class T> struct Group<SU3, T>
 		                               T(1.0 / 5040),
 		                               T(1.0 / 40320),
 		                               T(1.0 / 362880),
-		                               T(1.0 / 3628800)};
+		                               T(1.0 / 3628800),
+		                               T(1.0 / 39916800),
+		                               T(1.0 / 479001600),
+		                               T(1.0 / 6227020800),
+		                               T(1.0 / 87178291200),
+		                               T(1.0 / 1307674368000),
+		                               T(1.0 / 20922789888000),
+		                               T(1.0 / 355687428096000),
+		                               T(1.0 / 6402373705728000)};
 		cx<T> u0 = {inv_fact[N], T(0)}, u1 = {T(0), T(0)}, u2 = {T(0), T(0)};
 #pragma unroll
 		for (int k = N - 1; k >= 0; --k)
@@ -517,6 +602,23 @@ template <class T> struct Group<SU3, T>
 			u0 = n0;
 		}
 		E r;
+		if constexpr (sizeof(T) == 8)
+		{
+			// X_ii is imaginary and (X^2)_ii real: two fused multiply-adds a real part
+#pragma unroll
+			for (int i = 0; i < 3; ++i)
+#pragma unroll
+				for (int j = 0; j < 3; ++j)
+				{
+					cx<T> x = X.at(i, j), y = X2.at(i, j);
+					if (i == j)
+						r.set(i, j, {fma(u2.re, y.re, fma(-u1.im, x.im, u0.re)), fma(u2.im, y.re, fma(u1.re, x.im, u0.im))});
+					else
+						r.set(i, j, {fma(u1.re, x.re, fma(-u1.im, x.im, fma(u2.re, y.re, -u2.im * y.im))),
+						             fma(u1.re, x.im, fma(u1.im, x.re, fma(u2.re, y.im, u2.im * y.re)))});
+				}
+			return r;
+		}
 #pragma unroll
 		for (int i = 0; i < 3; ++i)
 #pragma unroll
@@ -622,18 +724,19 @@ template <class T> struct Group<SU3, T>
 			if (c1 < T(0.5))
 				return exp_series<10>(X, X2, c1, -c0);
 		}
-		cx<T> f0, f1, f2;
-		T const tiny = sizeof(T) == 8 ? T(1e-11) : T(1e-5);
-		if (c1 < tiny)
-		{
-			// exp(X) = 1 + X + X^2/2 + X^3/6; with X^3 = -i Q^3 and
-			// Q^3 = c1 Q + c0: 1 + X + X^2/2 - i (c1 Q + c0)/6
-			// -> f0 = 1 - i c0/6, f1 (on Q) = i - i c1/6, f2 (on Q^2) = -1/2
-			f0 = {T(1), -c0 * T(1.0 / 6.0)};
-			f1 = {T(0), T(1) - c1 * T(1.0 / 6.0)};
-			f2 = {T(-0.5), T(0)};
-		}
 		else
+		{
+			// the same series to FP64: the remainders are below 0.2^12/12! =
+			// 9e-18 for |X| < 0.2 and 1/19! = 8e-18 for |X| < 1. About 250
+			// operations against about 600 of the closed form below (three
+			// sincos, an acos, two square roots and two divisions), whose
+			// denominator also loses digits where two eigenvalues come close
+			if (c1 < T(0.02))
+				return exp_series<11>(X, X2, c1, -c0);
+			if (c1 < T(0.5))
+				return exp_series<18>(X, X2, c1, -c0);
+		}
+		cx<T> f0, f1, f2;
 		{
 			bool neg = c0 < T(0);
 			T c0a = neg ? -c0 : c0;
@@ -730,7 +833,29 @@ template <class T> struct Group<SU3, T>
 		}
 		else
 		{
-			E aa = mul_nd(a, a);
+			// a a^dagger is hermitian: the upper triangle (54 operations, not 108)
+			E aa;
+#pragma unroll
+			for (int i = 0; i < 3; ++i)
+#pragma unroll
+				for (int j = i; j < 3; ++j)
+				{
+					T re = T(0), im = T(0);
+#pragma unroll
+					for (int k = 0; k < 3; ++k)
+					{
+						cx<T> x = a.at(i, k), y = a.at(j, k);
+						re = k ? fma(x.re, y.re, re) : x.re * y.re;
+						re = fma(x.im, y.im, re);
+						if (j > i)
+						{
+							im = k ? fma(x.im, y.re, im) : x.im * y.re;
+							im = fma(-x.re, y.im, im);
+						}
+					}
+					aa.set(i, j, {re, im});
+					aa.set(j, i, {re, -im});
+				}
 			E aaa = mul(aa, a);
 #pragma unroll
 			for (int k = 0; k < 18; ++k)

@@ -280,7 +280,15 @@ template <class T> struct HbUpdate<SU3, T>
 			if (!(k > T(0)) || !su2_sample(T(2) * beta * k / T(3), rs, x))
 				continue;
 			T p[2], q[2];
-			times_vdag(x, a, b, k, p, q);
+			if constexpr (sizeof(T) == 8)
+			{
+				// one division, not four (an FP64 division is about 25 operations)
+				T rk = T(1) / k;
+				T an[2] = {a[0] * rk, a[1] * rk}, bn[2] = {b[0] * rk, b[1] * rk};
+				times_vdag(x, an, bn, T(1), p, q);
+			}
+			else
+				times_vdag(x, a, b, k, p, q);
 			left_mul(u, i, j, p, q);
 			left_mul(W, i, j, p, q);
 		}
@@ -295,13 +303,28 @@ template <class T> struct HbUpdate<SU3, T>
 			sub_rows(sg, i, j);
 			T a[2], b[2];
 			block(W, i, j, a, b);
-			T k = sqrt(a[0] * a[0] + a[1] * a[1] + b[0] * b[0] + b[1] * b[1]);
-			if (!(k > T(0)))
-				continue;
-			// R = (v^dagger)^2 = X v^dagger with X = v^dagger
-			T x[4] = {a[0] / k, -b[1] / k, -b[0] / k, -a[1] / k};
+			T n2 = a[0] * a[0] + a[1] * a[1] + b[0] * b[0] + b[1] * b[1];
 			T p[2], q[2];
-			times_vdag(x, a, b, k, p, q);
+			if constexpr (sizeof(T) == 8)
+			{
+				// R = (v^dagger)^2 = 2 Re(a) v^dagger / |v| - 1 for the unit v =
+				// (a, b) / |v| (Cayley-Hamilton): one division, no square root
+				if (!(n2 > T(0)))
+					continue;
+				T c = T(2) * a[0] / n2;
+				p[0] = fma(c, a[0], T(-1)), p[1] = -c * a[1];
+				q[0] = -c * b[0], q[1] = -c * b[1];
+			}
+			else
+			{
+				// R = (v^dagger)^2 = X v^dagger with X = v^dagger. FP32 keeps these
+				// roundings: a sweep amplifies a difference several times over
+				T k = sqrt(n2);
+				if (!(k > T(0)))
+					continue;
+				T x[4] = {a[0] / k, -b[1] / k, -b[0] / k, -a[1] / k};
+				times_vdag(x, a, b, k, p, q);
+			}
 			left_mul(u, i, j, p, q);
 			left_mul(W, i, j, p, q);
 		}

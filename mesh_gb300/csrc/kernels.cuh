@@ -545,6 +545,10 @@ template <> struct Prod<SU3, float, 1> : ProdF2
 {
 };
 
+// FP64 SU(3): sums of products run inside the products' fused multiply-add
+// chains (Group::add_nd and its kin), 18 FP64 adds less a product
+template <int GRP, class T> inline constexpr bool kAddChain = GRP == SU3 && sizeof(T) == 8;
+
 // staple sum for link (x, mu) in the reference's association and summation
 // order (utils.h:119-137): for nu = 0..Nd-1, nu != mu, the upper staple
 // U_nu(x+mu) (U_nu(x) U_mu(x+nu))^+ then the lower staple
@@ -568,14 +572,20 @@ __device__ __forceinline__ typename Group<GRP, T>::E staple(Geom const &g, Site<
 			E b = ld(nu, xpm);
 			E c = ld(mu, eo_shift1<ND>(g, st, nu, +1));
 			E d = ld(nu, s);
-			Gp::add_to(S, Pr::mul_nd(b, Pr::mul(d, c)));
+			if constexpr (kAddChain<GRP, T>)
+				Gp::add_nd(S, b, Pr::mul(d, c));
+			else
+				Gp::add_to(S, Pr::mul_nd(b, Pr::mul(d, c)));
 		}
 		{
 			int64_t y = eo_shift1<ND>(g, st, nu, -1);
 			E e = ld(mu, y);
 			E f = ld(nu, eo_shift2<ND>(g, st, nu, -1, mu, +1));
 			E h = ld(nu, y);
-			Gp::add_to(S, Pr::mul_dn(Pr::mul(e, f), h));
+			if constexpr (kAddChain<GRP, T>)
+				Gp::add_dn(S, Pr::mul(e, f), h);
+			else
+				Gp::add_to(S, Pr::mul_dn(Pr::mul(e, f), h));
 		}
 	}
 	return S;
@@ -1121,6 +1131,8 @@ __device__ __forceinline__ double site_md(Geom const &g, Site<ND> const &st, int
 				ef = Pr::mul(ld(mu, y), f);
 			if constexpr (F2 && GRP == SU3)
 				S = ProdF2::add_dn(S, ef, ld(nu, y));
+			else if constexpr (kAddChain<GRP, T>)
+				Gp::add_dn(S, ef, ld(nu, y));
 			else
 				Gp::add_to(S, Pr::mul_dn(ef, ld(nu, y)));
 		}
@@ -1369,6 +1381,23 @@ __global__ void __launch_bounds__(kBlock) k_reunit(int64_t n_total, int64_t V, T
 // Landau gauge fixing
 // ---------------------------------------------------------------------------
 
+// K += U_mu(x) g(x+mu)^+ + (g(x-mu) U_mu(x-mu))^+: the terms of direction mu
+// in the sum that multiplies g(x) in the gauge functional
+template <int GRP, class T, class E> __device__ __forceinline__ void add_closing(E &K, E const &u, E const &gf, E const &gb, E const &ub)
+{
+	using Gp = Group<GRP, T>;
+	if constexpr (GRP == SU3)
+	{
+		Gp::add_nd(K, u, gf);
+		Gp::add_mul_adj(K, gb, ub);
+	}
+	else
+	{
+		Gp::add_to(K, Gp::mul_nd(u, gf));
+		Gp::add_to(K, Gp::adj(Gp::mul(gb, ub)));
+	}
+}
+
 // sum_x sum_mu ReTr(g(x) U_mu(x) g(x+mu)^+)
 template <int GRP, class T, int ND>
 __global__ void __launch_bounds__(kBlock)
@@ -1464,8 +1493,7 @@ __global__ void __launch_bounds__(kBlock)
 			int64_t f = eo_shift1<ND>(g, st, mu, +1), b = eo_shift1<ND>(g, st, mu, -1);
 			Soa<T, Gp::NR>::load(G, g.V, f, gf.v);
 			Soa<T, Gp::NR>::load(G, g.V, b, gb.v);
-			Gp::add_to(d, Gp::mul_nd(ld(mu, s), gf));
-			Gp::add_to(d, Gp::adj(Gp::mul(gb, ld(mu, b))));
+			add_closing<GRP, T>(d, ld(mu, s), gf, gb, ld(mu, b));
 		}
 		E gx;
 		Soa<T, Gp::NR>::load(G, g.V, s, gx.v);
@@ -1551,11 +1579,11 @@ template <class T> struct OrUpdate<SU3, T>
 			for (int k = 0; k < 3; ++k)
 			{
 				cx<T> gi = gx.at(i, k), gj = gx.at(j, k);
-				gx.set(i, k, cadd(cmul(a, gi), cmul(b, gj)));
-				gx.set(j, k, cadd(cmul(c, gi), cmul(d, gj)));
+				gx.set(i, k, cmul2(a, gi, b, gj));
+				gx.set(j, k, cmul2(c, gi, d, gj));
 				cx<T> wi = W.at(i, k), wj = W.at(j, k);
-				W.set(i, k, cadd(cmul(a, wi), cmul(b, wj)));
-				W.set(j, k, cadd(cmul(c, wi), cmul(d, wj)));
+				W.set(i, k, cmul2(a, wi, b, wj));
+				W.set(j, k, cmul2(c, wi, d, wj));
 			}
 		}
 		return gx;
@@ -1582,9 +1610,7 @@ __global__ void __launch_bounds__(kBlock)
 			int64_t f = eo_shift1<ND>(g, st, mu, +1), b = eo_shift1<ND>(g, st, mu, -1);
 			Soa<T, Gp::NR>::load(G, g.V, f, gf.v);
 			Soa<T, Gp::NR>::load(G, g.V, b, gb.v);
-			Gp::add_to(K, Gp::mul_nd(ld(mu, s), gf));
-			// U_mu(x-mu)^+ g(x-mu)^+ = (g(x-mu) U_mu(x-mu))^+
-			Gp::add_to(K, Gp::adj(Gp::mul(gb, ld(mu, b))));
+			add_closing<GRP, T>(K, ld(mu, s), gf, gb, ld(mu, b));
 		}
 		E gx;
 		Soa<T, Gp::NR>::load(G, g.V, s, gx.v);
