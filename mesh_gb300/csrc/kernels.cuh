@@ -1425,85 +1425,97 @@ __global__ void __launch_bounds__(kBlock)
 	grid_sum<kBlock>(acc, out);
 }
 
-// Delta(x) = sum_mu [A_mu(x) - A_mu(x-mu)], A_mu(y) = proj(g(y) U_mu(y) g(y+mu)^+)
-template <int GRP, class T, int ND>
-__device__ __forceinline__ void divergence(Geom const &g, Site<ND> const &st, int64_t s, LinkLoad<GRP, T, ND> const &ld,
-                                           T const *__restrict__ G, T *D)
+// The kernels on K(x) = sum_mu U_mu(x) g(x+mu)^+ + (g(x-mu) U_mu(x-mu))^+ work
+// in blocks of 32 sites and one warp per direction: warp mu adds its two
+// products, the partial sums meet in shared memory, and warp 0 finishes the 32
+// sites. In FP64 (the solvers' precision) they are bound by the FP64 pipe,
+// which takes a warp instruction only every 16 cycles, so what counts is the
+// number of FP64 operations and that every SM gets the same share: a thread per
+// site gave a half sweep of 24^4 SU(3) 648 blocks of 256 (a last wave a third
+// full) and lattices of a few thousand sites a handful of busy SMs.
+template <int GRP, class T, int ND> struct ClosingSum
 {
 	using Gp = Group<GRP, T>;
 	using E = typename Gp::E;
-#pragma unroll
-	for (int k = 0; k < Gp::NA; ++k)
-		D[k] = T(0);
-	E gx;
-	Soa<T, Gp::NR>::load(G, g.V, s, gx.v);
-#pragma unroll
-	for (int mu = 0; mu < ND; ++mu)
-	{
-		E gf, gb, ub;
-		int64_t f = eo_shift1<ND>(g, st, mu, +1), b = eo_shift1<ND>(g, st, mu, -1);
-		Soa<T, Gp::NR>::load(G, g.V, f, gf.v);
-		Soa<T, Gp::NR>::load(G, g.V, b, gb.v);
-		T a[Gp::NA];
-		Gp::proj(Gp::mul_nd(Gp::mul(gx, ld(mu, s)), gf), a);
-#pragma unroll
-		for (int k = 0; k < Gp::NA; ++k)
-			D[k] += a[k];
-		Gp::proj(Gp::mul_nd(Gp::mul(gb, ld(mu, b)), gx), a);
-#pragma unroll
-		for (int k = 0; k < Gp::NA; ++k)
-			D[k] -= a[k];
-	}
-}
+	static constexpr int NT = 32 * ND;
+	T k[ND][Gp::NR][32];
 
-template <int GRP, class T, int ND>
-__global__ void __launch_bounds__(kBlock)
-    k_landau_theta(Geom g, T const *__restrict__ U, T const *__restrict__ G, RedSlot out)
-{
-	using Gp = Group<GRP, T>;
-	LinkLoad<GRP, T, ND> ld{U, g.V};
-	double acc = 0.0;
-	MESH_GRID_LOOP(s, g.V)
+	// K of the block's 32 sites (valid: this lane's site exists); the result in
+	// warp 0 only. Every thread of the block must call it.
+	__device__ __forceinline__ E sum(Geom const &g, bool valid, Site<ND> const &st, int64_t s,
+	                                 LinkLoad<GRP, T, ND> const &ld, T const *G)
 	{
-		Site<ND> st = site_from_eo<ND>(g, s);
-		T D[Gp::NA];
-		divergence<GRP, T, ND>(g, st, s, ld, G, D);
-		acc += double(Gp::kin(D));
-	}
-	grid_sum<kBlock>(acc, out);
-}
-
-// F(x) = proj(g(x) d(x)) * scale, d = sum_mu U_mu(x) g(x+mu)^+ + (g(x-mu) U_mu(x-mu))^+
-// (Landau::deriv, landau.h:52-65)
-template <int GRP, class T, int ND>
-__global__ void __launch_bounds__(kBlock)
-    k_landau_deriv(Geom g, T const *__restrict__ U, T const *__restrict__ G, T *__restrict__ F, T scale)
-{
-	using Gp = Group<GRP, T>;
-	using E = typename Gp::E;
-	LinkLoad<GRP, T, ND> ld{U, g.V};
-	MESH_GRID_LOOP(s, g.V)
-	{
-		Site<ND> st = site_from_eo<ND>(g, s);
-		E d = Gp::zero();
-#pragma unroll
-		for (int mu = 0; mu < ND; ++mu)
+		int mu = threadIdx.x >> 5, lane = threadIdx.x & 31;
+		E K = Gp::zero();
+		if (valid)
 		{
 			E gf, gb;
-			int64_t f = eo_shift1<ND>(g, st, mu, +1), b = eo_shift1<ND>(g, st, mu, -1);
-			Soa<T, Gp::NR>::load(G, g.V, f, gf.v);
+			int64_t b = eo_shift1<ND>(g, st, mu, -1);
+			Soa<T, Gp::NR>::load(G, g.V, eo_shift1<ND>(g, st, mu, +1), gf.v);
 			Soa<T, Gp::NR>::load(G, g.V, b, gb.v);
-			add_closing<GRP, T>(d, ld(mu, s), gf, gb, ld(mu, b));
+			add_closing<GRP, T>(K, ld(mu, s), gf, gb, ld(mu, b));
 		}
-		E gx;
-		Soa<T, Gp::NR>::load(G, g.V, s, gx.v);
-		T o[Gp::NA];
-		Gp::proj(Gp::mul(gx, d), o);
+		if (mu > 0)
+		{
 #pragma unroll
-		for (int k = 0; k < Gp::NA; ++k)
-			o[k] *= scale;
-		Soa<T, Gp::NA>::store(F, g.V, s, o);
+			for (int r = 0; r < Gp::NR; ++r)
+				k[mu][r][lane] = K.v[r];
+		}
+		__syncthreads();
+		if (mu == 0)
+		{
+#pragma unroll
+			for (int m = 1; m < ND; ++m)
+#pragma unroll
+				for (int r = 0; r < Gp::NR; ++r)
+					K.v[r] += k[m][r][lane];
+		}
+		return K;
 	}
+};
+
+// Delta(x) = sum_mu [A_mu(x) - A_mu(x-mu)], A_mu(y) = proj(g(y) U_mu(y) g(y+mu)^+).
+// proj(M^+) = -proj(M), so -A_mu(x-mu) = proj(g(x) (g(x-mu) U_mu(x-mu))^+) and
+// Delta(x) = proj(g(x) K(x)) for any matrices: 9 products a site where the A_mu
+// one by one take 16. THETA: sum_x |Delta(x)|^2 into out; DERIV: F = scale
+// Delta (Landau::deriv, landau.h:52-65).
+// 24^4 SU(3) FP64 on a GB300: theta took 1519 us from the A_mu with a thread per
+// site, 636 us here (1039 FP64 operations a site, the pipe 90% busy).
+template <int GRP, class T, int ND, bool THETA, bool DERIV>
+__global__ void __launch_bounds__(32 * ND)
+    k_landau_delta(Geom g, T const *__restrict__ U, T const *__restrict__ G, T *__restrict__ F, T scale, RedSlot out)
+{
+	using Gp = Group<GRP, T>;
+	using E = typename Gp::E;
+	__shared__ ClosingSum<GRP, T, ND> sm;
+	LinkLoad<GRP, T, ND> ld{U, g.V};
+	double acc = 0.0;
+	for (int64_t s0 = int64_t(blockIdx.x) * 32; s0 < g.V; s0 += int64_t(gridDim.x) * 32)
+	{
+		int64_t s = s0 + (threadIdx.x & 31);
+		bool valid = s < g.V;
+		Site<ND> st = site_from_eo<ND>(g, valid ? s : 0);
+		E K = sm.sum(g, valid, st, s, ld, G);
+		if (threadIdx.x < 32 && valid)
+		{
+			E gx;
+			Soa<T, Gp::NR>::load(G, g.V, s, gx.v);
+			T D[Gp::NA];
+			Gp::proj(Gp::mul(gx, K), D);
+			if constexpr (THETA)
+				acc += double(Gp::kin(D));
+			if constexpr (DERIV)
+			{
+#pragma unroll
+				for (int k = 0; k < Gp::NA; ++k)
+					D[k] *= scale;
+				Soa<T, Gp::NA>::store(F, g.V, s, D);
+			}
+		}
+		__syncthreads(); // the partial sums are read
+	}
+	if constexpr (THETA)
+		grid_sum<32 * ND>(acc, out);
 }
 
 // second-order binomial h^omega of a unit quaternion, renormalised
@@ -1590,28 +1602,24 @@ template <class T> struct OrUpdate<SU3, T>
 	}
 };
 
-// one checkerboard half-sweep of overrelaxation on the sites of `parity`
+// one checkerboard half-sweep of overrelaxation on the sites of `parity`, 32 a
+// block (K reads g only on the other parity). 24^4 SU(3) FP64 on a GB300: 403 us
+// (1365 FP64 operations a site, the pipe 92% busy)
 template <int GRP, class T, int ND>
-__global__ void __launch_bounds__(kBlock)
-    k_landau_or_half(Geom g, int parity, T omega, T const *__restrict__ U, T *__restrict__ G)
+__global__ void __launch_bounds__(32 * ND)
+    k_landau_or_half(Geom g, int parity, T omega, T const *__restrict__ U, T *G)
 {
 	using Gp = Group<GRP, T>;
 	using E = typename Gp::E;
+	__shared__ ClosingSum<GRP, T, ND> sm;
 	LinkLoad<GRP, T, ND> ld{U, g.V};
-	MESH_GRID_LOOP(h, g.Vh)
+	int64_t h = int64_t(blockIdx.x) * 32 + (threadIdx.x & 31);
+	bool valid = h < g.Vh;
+	int64_t s = int64_t(parity) * g.Vh + (valid ? h : 0);
+	Site<ND> st = site_from_eo<ND>(g, s);
+	E K = sm.sum(g, valid, st, s, ld, G);
+	if (threadIdx.x < 32 && valid)
 	{
-		int64_t s = int64_t(parity) * g.Vh + h;
-		Site<ND> st = site_from_eo<ND>(g, s);
-		E K = Gp::zero();
-#pragma unroll
-		for (int mu = 0; mu < ND; ++mu)
-		{
-			E gf, gb;
-			int64_t f = eo_shift1<ND>(g, st, mu, +1), b = eo_shift1<ND>(g, st, mu, -1);
-			Soa<T, Gp::NR>::load(G, g.V, f, gf.v);
-			Soa<T, Gp::NR>::load(G, g.V, b, gb.v);
-			add_closing<GRP, T>(K, ld(mu, s), gf, gb, ld(mu, b));
-		}
 		E gx;
 		Soa<T, Gp::NR>::load(G, g.V, s, gx.v);
 		E r = OrUpdate<GRP, T>::apply(Gp::mul(gx, K), gx, omega);
@@ -2511,24 +2519,33 @@ template <int GRP, class T, int ND> struct Ops
 		    U.geom, static_cast<T const *>(U.d), static_cast<T const *>(g.d), out);
 		MESH_LAUNCH_CHECK();
 	}
+	// 32 sites a block; the reductions walk them with at most 8 blocks per SM
+	static unsigned site_blocks(int64_t n) { return unsigned((n + 31) / 32); }
+	static unsigned red_site_blocks(Context const &c, int64_t n)
+	{
+		int64_t b = site_blocks(n), cap = int64_t(c.num_sms) * 8;
+		b = b < cap ? b : cap;
+		return unsigned(b < kMaxRedBlocks ? b : kMaxRedBlocks);
+	}
 	static void landau_theta(Field const &U, Field const &g, RedSlot out)
 	{
 		auto &c = *U.ctx;
-		k_landau_theta<GRP, T, ND><<<red_blocks(c, U.geom.V), kBlock, 0, c.stream>>>(
-		    U.geom, static_cast<T const *>(U.d), static_cast<T const *>(g.d), out);
+		k_landau_delta<GRP, T, ND, true, false><<<red_site_blocks(c, U.geom.V), 32 * ND, 0, c.stream>>>(
+		    U.geom, static_cast<T const *>(U.d), static_cast<T const *>(g.d), nullptr, T(0), out);
 		MESH_LAUNCH_CHECK();
 	}
 	static void landau_deriv(Field &F, Field const &U, Field const &g, double scale)
 	{
 		auto &c = *U.ctx;
-		k_landau_deriv<GRP, T, ND><<<blocks(c, U.geom.V), kBlock, 0, c.stream>>>(
-		    U.geom, static_cast<T const *>(U.d), static_cast<T const *>(g.d), static_cast<T *>(F.d), T(scale));
+		k_landau_delta<GRP, T, ND, false, true><<<site_blocks(U.geom.V), 32 * ND, 0, c.stream>>>(
+		    U.geom, static_cast<T const *>(U.d), static_cast<T const *>(g.d), static_cast<T *>(F.d), T(scale),
+		    RedSlot{});
 		MESH_LAUNCH_CHECK();
 	}
 	static void landau_or_half(Field const &U, Field &g, double omega, int parity)
 	{
 		auto &c = *U.ctx;
-		k_landau_or_half<GRP, T, ND><<<blocks(c, U.geom.Vh), kBlock, 0, c.stream>>>(
+		k_landau_or_half<GRP, T, ND><<<site_blocks(U.geom.Vh), 32 * ND, 0, c.stream>>>(
 		    U.geom, parity, T(omega), static_cast<T const *>(U.d), static_cast<T *>(g.d));
 		MESH_LAUNCH_CHECK();
 	}
