@@ -549,6 +549,35 @@ template <> struct Prod<SU3, float, 1> : ProdF2
 // chains (Group::add_nd and its kin), 18 FP64 adds less a product
 template <int GRP, class T> inline constexpr bool kAddChain = GRP == SU3 && sizeof(T) == 8;
 
+// S += the upper and the lower staple of link (x, mu) in the plane (mu, nu)
+template <int GRP, class T, int ND, bool F2, class LD>
+__device__ __forceinline__ void add_staples(typename Group<GRP, T>::E &S, Geom const &g, Site<ND> const &st, int64_t s,
+                                            int mu, int nu, int64_t xpm, LD const &ld)
+{
+	using Gp = Group<GRP, T>;
+	using E = typename Gp::E;
+	using Pr = Prod<GRP, T, F2>;
+	{
+		E b = ld(nu, xpm);
+		E c = ld(mu, eo_shift1<ND>(g, st, nu, +1));
+		E d = ld(nu, s);
+		if constexpr (kAddChain<GRP, T>)
+			Gp::add_nd(S, b, Pr::mul(d, c));
+		else
+			Gp::add_to(S, Pr::mul_nd(b, Pr::mul(d, c)));
+	}
+	{
+		int64_t y = eo_shift1<ND>(g, st, nu, -1);
+		E e = ld(mu, y);
+		E f = ld(nu, eo_shift2<ND>(g, st, nu, -1, mu, +1));
+		E h = ld(nu, y);
+		if constexpr (kAddChain<GRP, T>)
+			Gp::add_dn(S, Pr::mul(e, f), h);
+		else
+			Gp::add_to(S, Pr::mul_dn(Pr::mul(e, f), h));
+	}
+}
+
 // staple sum for link (x, mu) in the reference's association and summation
 // order (utils.h:119-137): for nu = 0..Nd-1, nu != mu, the upper staple
 // U_nu(x+mu) (U_nu(x) U_mu(x+nu))^+ then the lower staple
@@ -560,7 +589,6 @@ __device__ __forceinline__ typename Group<GRP, T>::E staple(Geom const &g, Site<
 {
 	using Gp = Group<GRP, T>;
 	using E = typename Gp::E;
-	using Pr = Prod<GRP, T, F2>;
 	E S = Gp::zero();
 	int64_t xpm = eo_shift1<ND>(g, st, mu, +1);
 #pragma unroll 1
@@ -568,25 +596,7 @@ __device__ __forceinline__ typename Group<GRP, T>::E staple(Geom const &g, Site<
 	{
 		if (nu == mu)
 			continue;
-		{
-			E b = ld(nu, xpm);
-			E c = ld(mu, eo_shift1<ND>(g, st, nu, +1));
-			E d = ld(nu, s);
-			if constexpr (kAddChain<GRP, T>)
-				Gp::add_nd(S, b, Pr::mul(d, c));
-			else
-				Gp::add_to(S, Pr::mul_nd(b, Pr::mul(d, c)));
-		}
-		{
-			int64_t y = eo_shift1<ND>(g, st, nu, -1);
-			E e = ld(mu, y);
-			E f = ld(nu, eo_shift2<ND>(g, st, nu, -1, mu, +1));
-			E h = ld(nu, y);
-			if constexpr (kAddChain<GRP, T>)
-				Gp::add_dn(S, Pr::mul(e, f), h);
-			else
-				Gp::add_to(S, Pr::mul_dn(Pr::mul(e, f), h));
-		}
+		add_staples<GRP, T, ND, F2>(S, g, st, s, mu, nu, xpm, ld);
 	}
 	return S;
 }
@@ -1232,6 +1242,64 @@ __global__ void __launch_bounds__(kBlock)
 	}
 }
 
+// The same update of FP64 SU(3) links in tiles of 32 links and one warp per plane:
+// warp w adds the two staples of its plane, the sums meet in shared memory and
+// warp 0 updates the 32 links. The FP64 pipe (a warp instruction every 16
+// cycles) is full with a few warps per SM, so the time is the FP64 operations
+// of the SM with the most tiles: half a direction of 12^3 x 24 is 81 blocks of
+// 256 links (half of the SMs idle) or 648 tiles. The grid is at most what is
+// resident at once and walks the tiles: a block for each tile gave the few
+// tiles past the first wave to the first SMs that finished, three at a time.
+// FP32 links keep the thread per link (k_gauge_update), whose order of
+// summation the sweeps' results depend on.
+// 12^3 x 24 SU(3) on a GB300, heat-bath / overrelaxation of half a direction:
+// 210 / 130 us a thread per link, 198 / 126 a block per tile, 144 / 99 here.
+template <int GRP, class T, int ND, bool OR>
+__global__ void __launch_bounds__(32 * (ND - 1), 5)
+    k_gauge_update_planes(Geom g, int ntiles, int mu, int parity, T *U, double beta, uint64_t seed, uint64_t ctr)
+{
+	using Gp = Group<GRP, T>;
+	using E = typename Gp::E;
+	__shared__ T sm[ND > 2 ? ND - 2 : 1][Gp::NR][32];
+	LinkLoad<GRP, T, ND> ld{U, g.V};
+	int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+	int nu = w < mu ? w : w + 1;
+	for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x)
+	{
+		int64_t i = int64_t(tile) * 32 + lane;
+		bool valid = i < g.Vh;
+		int64_t s = int64_t(parity) * g.Vh + (valid ? i : 0);
+		Site<ND> st = site_from_eo<ND>(g, s);
+		E S = Gp::zero();
+		if (valid)
+			add_staples<GRP, T, ND, false>(S, g, st, s, mu, nu, eo_shift1<ND>(g, st, mu, +1), ld);
+		if (w > 0)
+		{
+#pragma unroll
+			for (int r = 0; r < Gp::NR; ++r)
+				sm[w - 1][r][lane] = S.v[r];
+		}
+		__syncthreads();
+		if (w == 0 && valid)
+		{
+#pragma unroll
+			for (int k = 0; k < ND - 2; ++k)
+#pragma unroll
+				for (int r = 0; r < Gp::NR; ++r)
+					S.v[r] += sm[k][r][lane];
+			auto v = comp<T, Gp::NR>(U, g.V, mu);
+			E u;
+			v.load(s, u.v);
+			if constexpr (OR)
+				HbUpdate<GRP, T>::overrelax(u, S);
+			else
+				HbUpdate<GRP, T>::heatbath(u, S, T(beta), HbStream{seed, ctr, uint32_t(st.lex), uint32_t(mu), 0u});
+			v.store(s, u.v);
+		}
+		__syncthreads(); // the sums are read
+	}
+}
+
 // ---------------------------------------------------------------------------
 // Wilson loops (legacy src/old/mesh/wilson.cpp:40-75): straight lines of links
 // built one link at a time, then the rectangular loops from four lines
@@ -1732,6 +1800,16 @@ template <int GRP, class T, int ND> struct Ops
 	{
 		unsigned b = grid_for(c, n, kBlock, 4);
 		return b < unsigned(kMaxRedBlocks) ? b : unsigned(kMaxRedBlocks);
+	}
+
+	// grid of a kernel that walks `tiles` tiles: one block each, at most as many
+	// as are resident at once
+	template <class K> static unsigned resident_grid(Context const &c, K kernel, int threads, int64_t tiles)
+	{
+		int per_sm = 1;
+		MESH_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0));
+		int64_t cap = int64_t(c.num_sms) * (per_sm < 1 ? 1 : per_sm);
+		return unsigned(tiles < cap ? tiles : cap);
 	}
 
 	static void import_(Field &f, void const *stage)
@@ -2588,12 +2666,27 @@ template <int GRP, class T, int ND> struct Ops
 		for (int mu = 0; mu < ND; ++mu)
 			for (int par = 0; par < 2; ++par)
 			{
-				if (overrelax)
-					k_gauge_update<GRP, T, ND, true><<<blocks(c, U.geom.Vh), kBlock, 0, c.stream>>>(
-					    U.geom, mu, par, static_cast<T *>(U.d), beta, seed, ctr);
+				T *u = static_cast<T *>(U.d);
+				// U(1) and SU(2) staples are too few operations to bind the FP64 pipe
+				if constexpr (GRP == SU3 && sizeof(T) == 8)
+				{
+					int nt = int(site_blocks(U.geom.Vh));
+					constexpr int kThreads = 32 * (ND - 1);
+					if (overrelax)
+						k_gauge_update_planes<GRP, T, ND, true>
+						    <<<resident_grid(c, k_gauge_update_planes<GRP, T, ND, true>, kThreads, nt), kThreads, 0,
+						       c.stream>>>(U.geom, nt, mu, par, u, beta, seed, ctr);
+					else
+						k_gauge_update_planes<GRP, T, ND, false>
+						    <<<resident_grid(c, k_gauge_update_planes<GRP, T, ND, false>, kThreads, nt), kThreads, 0,
+						       c.stream>>>(U.geom, nt, mu, par, u, beta, seed, ctr);
+				}
+				else if (overrelax)
+					k_gauge_update<GRP, T, ND, true>
+					    <<<blocks(c, U.geom.Vh), kBlock, 0, c.stream>>>(U.geom, mu, par, u, beta, seed, ctr);
 				else
-					k_gauge_update<GRP, T, ND, false><<<blocks(c, U.geom.Vh), kBlock, 0, c.stream>>>(
-					    U.geom, mu, par, static_cast<T *>(U.d), beta, seed, ctr);
+					k_gauge_update<GRP, T, ND, false>
+					    <<<blocks(c, U.geom.Vh), kBlock, 0, c.stream>>>(U.geom, mu, par, u, beta, seed, ctr);
 				MESH_LAUNCH_CHECK();
 			}
 	}
