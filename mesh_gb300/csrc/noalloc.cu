@@ -92,7 +92,7 @@ void check_links(int device, void const *links)
 template <int GRP, class T, int ND>
 void launch(Geom const &g, void const *links, unsigned blocks, cudaStream_t st, RedSlot slot)
 {
-	k_plaquette<GRP, T, ND><<<blocks, kBlock, 0, st>>>(g, static_cast<T const *>(links), slot);
+	k_plaquette<GRP, T, ND><<<blocks, 32 * kPlanes<ND>, 0, st>>>(g, static_cast<T const *>(links), slot);
 }
 
 template <int GRP, class T>
@@ -138,11 +138,7 @@ extern "C" int mesh_plaquette_noalloc(int device, int group, int precision, int 
 		// the grid mesh_plaquette uses on this device (a function of the volume
 		// and the SM count only); a grid beyond the scratch is refused rather
 		// than shrunk, as a different grid would change the summation order
-		int64_t need = (V + kBlock - 1) / kBlock;
-		int64_t cap = int64_t(d.num_sms) * 4;
-		int64_t blocks = need < cap ? need : cap;
-		if (blocks > kMaxRedBlocks)
-			blocks = kMaxRedBlocks;
+		unsigned blocks = precision == MESH_F32 ? plaquette_grid<float>(d.num_sms, V) : plaquette_grid<double>(d.num_sms, V);
 		require(blocks <= kNoAllocMaxBlocks,
 		        "mesh_plaquette_noalloc: the reduction needs more blocks than MESH_NOALLOC_MAX_BLOCKS");
 		auto st = static_cast<cudaStream_t>(stream);
@@ -156,16 +152,16 @@ extern "C" int mesh_plaquette_noalloc(int device, int group, int precision, int 
 		switch (group)
 		{
 		case 1:
-			f32 ? launch_nd<1, float>(nd, g, links, unsigned(blocks), st, slot)
-			    : launch_nd<1, double>(nd, g, links, unsigned(blocks), st, slot);
+			f32 ? launch_nd<1, float>(nd, g, links, blocks, st, slot)
+			    : launch_nd<1, double>(nd, g, links, blocks, st, slot);
 			break;
 		case 2:
-			f32 ? launch_nd<2, float>(nd, g, links, unsigned(blocks), st, slot)
-			    : launch_nd<2, double>(nd, g, links, unsigned(blocks), st, slot);
+			f32 ? launch_nd<2, float>(nd, g, links, blocks, st, slot)
+			    : launch_nd<2, double>(nd, g, links, blocks, st, slot);
 			break;
 		default:
-			f32 ? launch_nd<3, float>(nd, g, links, unsigned(blocks), st, slot)
-			    : launch_nd<3, double>(nd, g, links, unsigned(blocks), st, slot);
+			f32 ? launch_nd<3, float>(nd, g, links, blocks, st, slot)
+			    : launch_nd<3, double>(nd, g, links, blocks, st, slot);
 			break;
 		}
 		MESH_LAUNCH_CHECK();

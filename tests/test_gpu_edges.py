@@ -48,3 +48,11 @@ def test_fp64_su3_sweeps(ctx, oracle, dims, overrelax):
         mg.heatbath_sweep(U, 2.0 * g, 21, 3)
     ref = oracle.gauge_sweep(g, 2, dims, U64, 2.0 * g, 21, 3, overrelax=overrelax)
     assert rel(U.export(), ref) < 1e-11
+
+
+@pytest.mark.parametrize("dims", SHAPES, ids=lambda d: "x".join(map(str, d)))
+@pytest.mark.parametrize("g,p", [(1, 2), (2, 2), (3, 2), (3, 1)])
+def test_plaquette_tiles(ctx, oracle, g, p, dims):
+    U64 = links(oracle, g, dims)
+    U = mg.GaugeField(ctx, g, p, mg.Grid(dims)).import_(U64.astype(mg.real_dtype(p)))
+    assert mg.plaquette(U) == pytest.approx(oracle.plaquette(g, 2, dims, U64), abs=1e-13 if p == 2 else 1e-6)
