@@ -40,6 +40,8 @@ void teardown_ctx(Context &c)
 	cudaFree(c.d_err);
 	if (c.d_stage)
 		cudaFree(c.d_stage);
+	if (c.d_md)
+		cudaFree(c.d_md);
 	if (c.own_stream && c.stream)
 		cudaStreamDestroy(c.stream);
 }
@@ -243,6 +245,38 @@ std::vector<double> make_deltas(std::string const &scheme, double epsilon, int s
 	return d;
 }
 
+bool capturing(Context const &c)
+{
+	cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+	return cudaStreamIsCapturing(c.stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone;
+}
+
+// the context's momentum-step scratch for U's lattice. Empty (the step then
+// runs without it) while the stream is being captured, as a later lattice may
+// replace the memory a captured launch points to, and when there is no memory.
+MdScratch ctx_md_scratch(Field const &U)
+{
+	Context &c = *U.ctx;
+	size_t need = ops_for(U).md_scratch_bytes(U.geom);
+	if (need == 0 || capturing(c))
+		return {};
+	if (c.md_bytes < need)
+	{
+		MESH_CUDA(cudaStreamSynchronize(c.stream));
+		cudaFree(c.d_md);
+		c.d_md = nullptr;
+		c.md_bytes = 0;
+		if (cudaMalloc(&c.d_md, need) != cudaSuccess)
+		{
+			cudaGetLastError();
+			c.d_md = nullptr;
+			return {};
+		}
+		c.md_bytes = need;
+	}
+	return {c.d_md, c.md_bytes};
+}
+
 void check_deltas(double const *deltas, int n)
 {
 	require(deltas != nullptr && n >= 1, "empty step table");
@@ -286,6 +320,8 @@ struct mesh_hmc_s
 	int *d_flag = nullptr;
 	int64_t count = 0; // trajectories enqueued
 	bool S_valid = false;
+	// products of a momentum step (allocated by the first step outside a capture)
+	MdScratch scratch;
 	// cached CUDA graph of one trajectory
 	cudaGraphExec_t graph = nullptr;
 	double graph_beta = 0;
@@ -331,6 +367,22 @@ struct mesh_hmc_s
 		drop_graph();
 	}
 
+	// the chain's scratch, before its first step; a chain without the memory
+	// for it steps without it
+	void ensure_scratch()
+	{
+		size_t need = ops_for(U.f).md_scratch_bytes(U.f.geom);
+		if (need == 0 || scratch.d || capturing(*ctx))
+			return;
+		if (cudaMalloc(&scratch.d, need) == cudaSuccess)
+			scratch.bytes = need;
+		else
+		{
+			cudaGetLastError();
+			scratch.d = nullptr;
+		}
+	}
+
 	// Enqueue one trajectory (runHmcUpdate, hmc.cpp:73-107) on the stream.
 	// P0 != nullptr: supplied momenta; uniform NaN: draw from the stream.
 	void enqueue(double beta, double const *deltas, int n, Field const *P0, double uniform)
@@ -338,6 +390,7 @@ struct mesh_hmc_s
 		Field &u = U.f, &un = Unew.f, &p = P.f;
 		auto const &ops = ops_for(u);
 		Context &c = *ctx;
+		ensure_scratch();
 		if (!S_valid)
 		{
 			ops.hmc_plaquette(u, rs(S_CUR));
@@ -363,13 +416,13 @@ struct mesh_hmc_s
 			{
 				RedSlot kin = rs(K_NEW);
 				RedSlot *k = i == last_p ? &kin : nullptr;
-				if (i + 1 < n && ops.hmc_md_step(p, *cur, *spare, coef0 * deltas[i], deltas[i + 1], i + 1 == n - 1, k))
+				if (i + 1 < n && ops.hmc_md_step(p, *cur, *spare, coef0 * deltas[i], deltas[i + 1], i + 1 == n - 1, k, scratch))
 				{
 					std::swap(cur, spare);
 					++i; // the link update i + 1 is done
 				}
 				else
-					ops.hmc_momentum_step(p, *cur, coef0 * deltas[i], k);
+					ops.hmc_momentum_step(p, *cur, coef0 * deltas[i], k, scratch);
 			}
 		}
 		if (last_p < 0)
@@ -952,7 +1005,7 @@ int mesh_momentum_step(mesh_field Ph, mesh_field Uh, double beta, double delta)
 		same_shape(U, P);
 		require(P.kind == MESH_ALGEBRA && P.nstack == U.nstack, "momenta must be an algebra field like U");
 		DeviceGuard dg(U.ctx->device);
-		ops_for(U).momentum_step(P, U, beta / (2.0 * group_nc(U.group)) * delta, nullptr);
+		ops_for(U).momentum_step(P, U, beta / (2.0 * group_nc(U.group)) * delta, nullptr, ctx_md_scratch(U));
 	});
 }
 
@@ -967,11 +1020,12 @@ int mesh_run_hmd(mesh_field Uh, mesh_field Ph, double beta, double const *deltas
 		DeviceGuard dg(U.ctx->device);
 		auto const &ops = ops_for(U);
 		double coef0 = beta / (2.0 * group_nc(U.group));
+		MdScratch scratch = ctx_md_scratch(U);
 		for (int i = 0; i < n; ++i)
 			if (i % 2 == 0)
 				ops.evolve(U, U, P, deltas[i], false);
 			else
-				ops.momentum_step(P, U, coef0 * deltas[i], nullptr);
+				ops.momentum_step(P, U, coef0 * deltas[i], nullptr, scratch);
 	});
 }
 
@@ -1039,6 +1093,7 @@ int mesh_hmc_destroy(mesh_hmc h)
 		cudaFree(h->d_hist);
 		cudaFree(h->d_flag);
 		cudaFree(h->d_part);
+		cudaFree(h->scratch.d);
 		cudaFree(h->d_res);
 		cudaFree(h->d_cnt);
 		// the fields hold the chain's references to the context
@@ -1128,7 +1183,8 @@ int mesh_hmc_momentum_step(mesh_hmc h, double beta, double delta)
 		require(h != nullptr, "null hmc");
 		DeviceGuard dg(h->ctx->device);
 		Field &U = h->U.f, &P = h->P.f;
-		ops_for(U).hmc_momentum_step(P, U, beta / (2.0 * group_nc(U.group)) * delta, nullptr);
+		h->ensure_scratch();
+		ops_for(U).hmc_momentum_step(P, U, beta / (2.0 * group_nc(U.group)) * delta, nullptr, h->scratch);
 	});
 }
 
@@ -1139,8 +1195,9 @@ int mesh_hmc_md_step(mesh_hmc h, double beta, double dp, double du)
 		DeviceGuard dg(h->ctx->device);
 		Field &U = h->U.f, &P = h->P.f;
 		auto const &ops = ops_for(U);
+		h->ensure_scratch();
 		double coef = beta / (2.0 * group_nc(U.group)) * dp;
-		if (ops.hmc_md_step(P, U, h->Ut.f, coef, du, false, nullptr))
+		if (ops.hmc_md_step(P, U, h->Ut.f, coef, du, false, nullptr, h->scratch))
 		{
 			// the new links are in Ut: swap the buffers (a captured trajectory
 			// holds the old addresses, so it is dropped)
@@ -1149,7 +1206,7 @@ int mesh_hmc_md_step(mesh_hmc h, double beta, double dp, double du)
 		}
 		else
 		{
-			ops.hmc_momentum_step(P, U, coef, nullptr);
+			ops.hmc_momentum_step(P, U, coef, nullptr, h->scratch);
 			ops.hmc_evolve(U, U, P, du, false);
 		}
 		h->S_valid = false;
@@ -1221,9 +1278,14 @@ int mesh_hmc_run(mesh_hmc h, double beta, double const *deltas, int n, int count
 			ops_for(h->U.f).hmc_plaquette(h->U.f, h->rs(mesh_hmc_s::S_CUR));
 			h->S_valid = true;
 		}
-		// choose launch variants before capturing (tuning times kernels)
-		ops_for(h->U.f).hmc_tune(h->P.f, h->Unew.f);
-		ops_for(h->U.f).hmc_tune_md(h->P.f, h->Unew.f, h->Ut.f);
+		h->ensure_scratch();
+		// choose launch variants before capturing (tuning times kernels); the
+		// step from stored products has none
+		if (!h->scratch.d || force_override() >= 0)
+		{
+			ops_for(h->U.f).hmc_tune(h->P.f, h->Unew.f);
+			ops_for(h->U.f).hmc_tune_md(h->P.f, h->Unew.f, h->Ut.f);
+		}
 		std::vector<double> dv(deltas, deltas + n);
 		if (!h->graph || h->graph_beta != beta || h->graph_deltas != dv || h->graph_hist != h->d_hist)
 		{

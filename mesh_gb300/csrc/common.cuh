@@ -63,6 +63,11 @@ struct Context
 	void *d_stage = nullptr;
 	size_t stage_bytes = 0;
 
+	// scratch of the momentum step on plain fields (md_products.cuh), grown on
+	// demand up to that file's cap
+	void *d_md = nullptr;
+	size_t md_bytes = 0;
+
 	void *stage(size_t bytes)
 	{
 		if (bytes > stage_bytes)

@@ -75,6 +75,14 @@ enum SlotId
 	SLOT_TMP2 = 1,
 };
 
+// device memory for the products of a momentum step (md_products.cuh): owned by
+// a chain (a captured trajectory holds its address) or by a context
+struct MdScratch
+{
+	void *d = nullptr;
+	size_t bytes = 0;
+};
+
 struct OpsTable
 {
 	// fields
@@ -95,7 +103,8 @@ struct OpsTable
 	void (*wilson_deriv)(Field &F, Field const &U, int mu, double beta);
 	void (*reunitize)(Field &U);
 	void (*evolve)(Field const &Usrc, Field &Udst, Field const &P, double t, bool reunit);
-	void (*momentum_step)(Field &P, Field const &U, double coef, RedSlot *kin);
+	// (scratch: md_scratch_bytes, or empty for the kernels without it)
+	void (*momentum_step)(Field &P, Field const &U, double coef, RedSlot *kin, MdScratch const &scratch);
 	// Landau
 	void (*landau_functional)(Field const &U, Field const &g, RedSlot out);
 	void (*landau_theta)(Field const &U, Field const &g, RedSlot out);
@@ -113,13 +122,14 @@ struct OpsTable
 	// and 1, row 2 rebuilt); the same as the generic ones otherwise
 	void (*hmc_plaquette)(Field const &U, RedSlot out);
 	void (*hmc_evolve)(Field const &Usrc, Field &Udst, Field const &P, double t, bool reunit);
-	void (*hmc_momentum_step)(Field &P, Field const &U, double coef, RedSlot *kin);
+	void (*hmc_momentum_step)(Field &P, Field const &U, double coef, RedSlot *kin, MdScratch const &scratch);
 	void (*hmc_tune)(Field &P, Field const &U);
 	// the trajectory's momentum step fused with the link update after it:
 	// P -= coef F(Uin), Uout = exp(tu P) Uin (reunitised when `reunit`);
 	// returns false, launching nothing, where the fused kernel does not apply
 	// (then the two steps run separately)
-	bool (*hmc_md_step)(Field &P, Field const &Uin, Field &Uout, double coef, double tu, bool reunit, RedSlot *kin);
+	bool (*hmc_md_step)(Field &P, Field const &Uin, Field &Uout, double coef, double tu, bool reunit, RedSlot *kin,
+	                    MdScratch const &scratch);
 	void (*hmc_tune_md)(Field &P, Field const &Uin, Field &Uout);
 	// Wilson loops (4D): Lout = Lprev U_dir(x + (n-1) dir); sum of the r x t loops
 	void (*line_extend)(Field const &U, int dir, int n, void const *Lprev, void *Lout);
@@ -129,6 +139,8 @@ struct OpsTable
 	// layout conversion reading / writing a device-accessible host buffer directly
 	void (*import_direct)(Field &f, void const *host);
 	void (*export_direct)(Field const &f, void *host);
+	// bytes of scratch the momentum step runs with on this lattice (0: none)
+	size_t (*md_scratch_bytes)(Geom const &g);
 };
 
 // autotuning registry (tune.cu): variant index per kernel/lattice key

@@ -561,7 +561,7 @@ template <class T> struct Group<SU3, T>
 	}
 	// exp(X) for antihermitian traceless X with |X| < 1 (Frobenius norm), as
 	// the power series truncated after X^N (N = 10: remainder below
-	// |X|^11/11! = 2.5e-8; N = 6 for |X| < 0.2: below 0.2^7/7! = 2.5e-9; FP64: N = 18 and 11) and
+	// |X|^11/11! = 2.5e-8; N = 6 for |X| < 0.2: below 0.2^7/7! = 2.5e-9) and
 	// reduced to a polynomial u0 + u1 X + u2 X^2 with the Cayley-Hamilton
 	// relation X^3 = -c1 X + i dim, c1 = |X|^2/2, i dim = det X; the series
 	// is summed by Horner's rule on the three coefficients (M. Luscher,
@@ -569,9 +569,9 @@ template <class T> struct Group<SU3, T>
 	// the FP32 trajectory's link update.
 	template <int N = 10> MESH_HD static E exp_series(E const &X, E const &X2, T c1, T dim)
 	{
-		static_assert(N >= 1 && N <= 18, "series order");
+		static_assert(N >= 1 && N <= 10, "series order");
 		// 1/k! for k = 0..N
-		constexpr T inv_fact[19] = {T(1),
+		constexpr T inv_fact[11] = {T(1),
 		                               T(1),
 		                               T(1.0 / 2),
 		                               T(1.0 / 6),
@@ -581,15 +581,7 @@ template <class T> struct Group<SU3, T>
 		                               T(1.0 / 5040),
 		                               T(1.0 / 40320),
 		                               T(1.0 / 362880),
-		                               T(1.0 / 3628800),
-		                               T(1.0 / 39916800),
-		                               T(1.0 / 479001600),
-		                               T(1.0 / 6227020800),
-		                               T(1.0 / 87178291200),
-		                               T(1.0 / 1307674368000),
-		                               T(1.0 / 20922789888000),
-		                               T(1.0 / 355687428096000),
-		                               T(1.0 / 6402373705728000)};
+		                               T(1.0 / 3628800)};
 		cx<T> u0 = {inv_fact[N], T(0)}, u1 = {T(0), T(0)}, u2 = {T(0), T(0)};
 #pragma unroll
 		for (int k = N - 1; k >= 0; --k)
@@ -602,23 +594,6 @@ template <class T> struct Group<SU3, T>
 			u0 = n0;
 		}
 		E r;
-		if constexpr (sizeof(T) == 8)
-		{
-			// X_ii is imaginary and (X^2)_ii real: two fused multiply-adds a real part
-#pragma unroll
-			for (int i = 0; i < 3; ++i)
-#pragma unroll
-				for (int j = 0; j < 3; ++j)
-				{
-					cx<T> x = X.at(i, j), y = X2.at(i, j);
-					if (i == j)
-						r.set(i, j, {fma(u2.re, y.re, fma(-u1.im, x.im, u0.re)), fma(u2.im, y.re, fma(u1.re, x.im, u0.im))});
-					else
-						r.set(i, j, {fma(u1.re, x.re, fma(-u1.im, x.im, fma(u2.re, y.re, -u2.im * y.im))),
-						             fma(u1.re, x.im, fma(u1.im, x.re, fma(u2.re, y.im, u2.im * y.re)))});
-				}
-			return r;
-		}
 #pragma unroll
 		for (int i = 0; i < 3; ++i)
 #pragma unroll
@@ -629,6 +604,74 @@ template <class T> struct Group<SU3, T>
 					z = cadd(z, u0);
 				r.set(i, j, z);
 			}
+		return r;
+	}
+	// The same series in FP64 on the packed element x (|X|^2 = 2 c1) for |X| < 1:
+	// N = 18, remainder below 1/19! = 8e-18. One order for all: a second one for
+	// smaller |X| saves 16 of 170 operations, but the links of a warp fall on both
+	// sides of any bound, and the warp then runs both series.
+	// X_ii = i a_i and (X^2)_ii real, X^2 hermitian, with a2 = -(a0 + a1):
+	//   (X^2)_01 = -i a2 b01 - b02 b12^*,  (X^2)_02 = -i a1 b02 + b01 b12,
+	//   (X^2)_12 = -i a0 b12 - b01^* b02,
+	//   det X = i (a0 |b12|^2 + a1 |b02|^2 + a2 |b01|^2 - a0 a1 a2 - 2 Im b01 b12 b02^*).
+	// About 170 operations; the closed form of exp_alg takes about 600 (three
+	// sincos, an acos, square roots, divisions), and its denominator loses
+	// digits where two eigenvalues come close.
+	MESH_HD static E exp_series_packed(T const *x, T n01, T n02, T n12, T c1)
+	{
+		constexpr int N = 18;
+		constexpr T inv_fact[N + 1] = {T(1),
+		                            T(1),
+		                            T(1.0 / 2),
+		                            T(1.0 / 6),
+		                            T(1.0 / 24),
+		                            T(1.0 / 120),
+		                            T(1.0 / 720),
+		                            T(1.0 / 5040),
+		                            T(1.0 / 40320),
+		                            T(1.0 / 362880),
+		                            T(1.0 / 3628800),
+		                            T(1.0 / 39916800),
+		                            T(1.0 / 479001600),
+		                            T(1.0 / 6227020800),
+		                            T(1.0 / 87178291200),
+		                            T(1.0 / 1307674368000),
+		                            T(1.0 / 20922789888000),
+		                            T(1.0 / 355687428096000),
+		                            T(1.0 / 6402373705728000)};
+		T a[3] = {x[0], x[1], -(x[0] + x[1])};
+		cx<T> b01 = {x[2], x[3]}, b02 = {x[4], x[5]}, b12 = {x[6], x[7]};
+		T d[3] = {-(fma(a[0], a[0], n01) + n02), -(fma(a[1], a[1], n01) + n12), -(fma(a[2], a[2], n02) + n12)};
+		cx<T> q01 = {fma(a[2], b01.im, fma(-b02.re, b12.re, -b02.im * b12.im)),
+		             fma(-a[2], b01.re, fma(b02.re, b12.im, -b02.im * b12.re))};
+		cx<T> w = {fma(b01.re, b12.re, -b01.im * b12.im), fma(b01.re, b12.im, b01.im * b12.re)};
+		cx<T> q02 = {fma(a[1], b02.im, w.re), fma(-a[1], b02.re, w.im)};
+		cx<T> q12 = {fma(a[0], b12.im, fma(-b01.re, b02.re, -b01.im * b02.im)),
+		             fma(-a[0], b12.re, fma(-b01.re, b02.im, b01.im * b02.re))};
+		T dim = fma(a[0], fma(-a[1], a[2], n12), fma(a[1], n02, a[2] * n01));
+		dim = fma(T(-2) * w.im, b02.re, fma(T(2) * w.re, b02.im, dim));
+		cx<T> u0 = {inv_fact[N], T(0)}, u1 = {T(0), T(0)}, u2 = {T(0), T(0)};
+#pragma unroll
+		for (int k = N - 1; k >= 0; --k)
+		{
+			cx<T> n0 = {fma(-dim, u2.im, inv_fact[k]), dim * u2.re};
+			cx<T> n1 = {fma(-c1, u2.re, u0.re), fma(-c1, u2.im, u0.im)};
+			u2 = u1;
+			u1 = n1;
+			u0 = n0;
+		}
+		E r;
+#pragma unroll
+		for (int i = 0; i < 3; ++i)
+			r.set(i, i, {fma(u2.re, d[i], fma(-u1.im, a[i], u0.re)), fma(u2.im, d[i], fma(u1.re, a[i], u0.im))});
+		// u1 X_ij + u2 (X^2)_ij, and for ji: X_ji = -X_ij^*, (X^2)_ji = (X^2)_ij^*
+		auto off = [&](int i, int j, cx<T> b, cx<T> q) {
+			r.set(i, j, cmul2(u1, b, u2, q));
+			r.set(j, i, cmul2(u1, cx<T>{-b.re, b.im}, u2, cx<T>{q.re, -q.im}));
+		};
+		off(0, 1, b01, q01);
+		off(0, 2, b02, q02);
+		off(1, 2, b12, q12);
 		return r;
 	}
 	// rows 0 and 1 of exp(t X) for X = from_alg(o), FP32, when |tX| < 0.2
@@ -711,6 +754,14 @@ template <class T> struct Group<SU3, T>
 #pragma unroll
 		for (int k = 0; k < 8; ++k)
 			x[k] = o[k] * t;
+		if constexpr (sizeof(T) == 8)
+		{
+			T n01 = fma(x[2], x[2], x[3] * x[3]), n02 = fma(x[4], x[4], x[5] * x[5]);
+			T n12 = fma(x[6], x[6], x[7] * x[7]), a2 = x[0] + x[1];
+			T h = fma(T(0.5), fma(x[0], x[0], fma(x[1], x[1], a2 * a2)), n01 + n02 + n12);
+			if (h < T(0.5))
+				return exp_series_packed(x, n01, n02, n12, h);
+		}
 		E X = from_alg(x);
 		E X2 = sq_ah(X);
 		// c1 = Tr(Q^2)/2 = |X|^2/2,  c0 = det(Q) = det(-iX) = -Im det(X)
@@ -723,18 +774,6 @@ template <class T> struct Group<SU3, T>
 				return exp_series<6>(X, X2, c1, -c0);
 			if (c1 < T(0.5))
 				return exp_series<10>(X, X2, c1, -c0);
-		}
-		else
-		{
-			// the same series to FP64: the remainders are below 0.2^12/12! =
-			// 9e-18 for |X| < 0.2 and 1/19! = 8e-18 for |X| < 1. About 250
-			// operations against about 600 of the closed form below (three
-			// sincos, an acos, two square roots and two divisions), whose
-			// denominator also loses digits where two eigenvalues come close
-			if (c1 < T(0.02))
-				return exp_series<11>(X, X2, c1, -c0);
-			if (c1 < T(0.5))
-				return exp_series<18>(X, X2, c1, -c0);
 		}
 		cx<T> f0, f1, f2;
 		{

@@ -264,8 +264,8 @@ __global__ void __launch_bounds__(kBlock)
 }
 
 // Gaussian momenta; also sums the kinetic energy norm2(P) in FP64
-template <int GRP, class T, int ND>
-__global__ void __launch_bounds__(kBlock)
+template <int GRP, class T, int ND, int BLOCK = kBlock>
+__global__ void __launch_bounds__(BLOCK)
     k_random_alg(Geom g, int nstack, uint64_t seed, uint64_t const *counter_dev, uint64_t counter, T *__restrict__ dev,
                  RedSlot kin)
 {
@@ -285,7 +285,7 @@ __global__ void __launch_bounds__(kBlock)
 		acc += double(Gp::kin(o));
 	}
 	if (kin.result)
-		grid_sum<kBlock>(acc, kin);
+		grid_sum<BLOCK>(acc, kin);
 }
 
 // sum over all components of the (kinetic) norm2
@@ -1804,6 +1804,7 @@ __global__ void __launch_bounds__(kBlock) k_gauge_transform(Geom g, T *__restric
 
 } // namespace meshgb
 #include "md_line.cuh"
+#include "md_products.cuh"
 namespace meshgb {
 
 // ---------------------------------------------------------------------------
@@ -1903,17 +1904,30 @@ template <int GRP, class T, int ND> struct Ops
 			                                                                  static_cast<T *>(f.d));
 		}
 		else
-			k_random_alg<GRP, T, ND><<<red_blocks(c, n), kBlock, 0, c.stream>>>(
-			    f.geom, f.nstack, seed, nullptr, counter, static_cast<T *>(f.d), kin);
+			launch_random_alg(f, seed, nullptr, counter, kin);
+		MESH_LAUNCH_CHECK();
+	}
+	// threads a block of the element-wise FP64 kernels: their time is the FP64
+	// instructions of the SM with the most warps, so small blocks spread small
+	// lattices (8^4 SU(3): 256 blocks of 64, where 64 blocks of 256 left 88 of 152
+	// SMs idle; momentum refresh 27.9 -> 17.9 us, link update 21.4 -> 12.9 us)
+	static constexpr int kElemBlock = sizeof(T) == 8 ? 64 : kBlock;
+	static unsigned elem_blocks(Context const &c, int64_t n, int per_sm)
+	{
+		unsigned b = grid_for(c, n, kElemBlock, per_sm * (kBlock / kElemBlock));
+		return b < unsigned(kMaxRedBlocks) ? b : unsigned(kMaxRedBlocks);
+	}
+	static void launch_random_alg(Field &f, uint64_t seed, uint64_t const *counter_dev, uint64_t counter, RedSlot kin)
+	{
+		auto &c = *f.ctx;
+		int64_t n = int64_t(f.nstack) * f.geom.V;
+		k_random_alg<GRP, T, ND, kElemBlock><<<elem_blocks(c, n, 4), kElemBlock, 0, c.stream>>>(
+		    f.geom, f.nstack, seed, counter_dev, counter, static_cast<T *>(f.d), kin);
 		MESH_LAUNCH_CHECK();
 	}
 	static void random_momenta_dev(Field &f, uint64_t seed, uint64_t const *counter_dev, RedSlot kin)
 	{
-		auto &c = *f.ctx;
-		int64_t n = int64_t(f.nstack) * f.geom.V;
-		k_random_alg<GRP, T, ND><<<red_blocks(c, n), kBlock, 0, c.stream>>>(f.geom, f.nstack, seed, counter_dev, 0,
-		                                                                  static_cast<T *>(f.d), kin);
-		MESH_LAUNCH_CHECK();
+		launch_random_alg(f, seed, counter_dev, 0, kin);
 	}
 	static void norm2(Field const &f, RedSlot out)
 	{
@@ -2021,11 +2035,11 @@ template <int GRP, class T, int ND> struct Ops
 		auto &c = *Udst.ctx;
 		int64_t n = int64_t(Udst.nstack) * Udst.geom.V;
 		if (reunit)
-			k_evolve<GRP, T, true><<<blocks(c, n), kBlock, 0, c.stream>>>(
+			k_evolve<GRP, T, true><<<elem_blocks(c, n, 8), kElemBlock, 0, c.stream>>>(
 			    n, Udst.geom.V, static_cast<T const *>(Usrc.d), static_cast<T *>(Udst.d),
 			    static_cast<T const *>(P.d), T(t));
 		else
-			k_evolve<GRP, T, false><<<blocks(c, n), kBlock, 0, c.stream>>>(
+			k_evolve<GRP, T, false><<<elem_blocks(c, n, 8), kElemBlock, 0, c.stream>>>(
 			    n, Udst.geom.V, static_cast<T const *>(Usrc.d), static_cast<T *>(Udst.d),
 			    static_cast<T const *>(P.d), T(t));
 		MESH_LAUNCH_CHECK();
@@ -2390,6 +2404,63 @@ template <int GRP, class T, int ND> struct Ops
 		b = unsigned(ts.ntiles < cap ? ts.ntiles : cap);
 		return ts;
 	}
+	// ---- FP64 SU(3): momentum step from stored products (md_products.cuh) -----
+	static constexpr bool kProducts = GRP == SU3 && sizeof(T) == 8;
+	static size_t md_scratch_bytes(Geom const &g)
+	{
+		size_t bytes = 0;
+		if constexpr (kProducts)
+			md_ring<T, ND>(g, &bytes);
+		return bytes;
+	}
+	// false (nothing launched) without scratch or with a pinned launch variant
+	static bool products_step(Field &P, Field const &U, Field *Uout, double coef, double tu, bool reunit, RedSlot *kin,
+	                          MdScratch const &scratch)
+	{
+		if constexpr (kProducts)
+		{
+			Geom const &g = U.geom;
+			size_t bytes = 0;
+			MdRing ring = md_ring<T, ND>(g, &bytes);
+			if (!scratch.d || scratch.bytes < bytes || force_override() >= 0)
+				return false;
+			auto &c = *U.ctx;
+			T *W = static_cast<T *>(scratch.d), *A = W + 2 * kPlanes<ND> * Gp::NR * ring.V;
+			T const *u = static_cast<T const *>(U.d);
+			T *p = static_cast<T *>(P.d), *uo = Uout ? static_cast<T *>(Uout->d) : nullptr;
+			auto products = [&](int x0, int n, int t0) {
+				auto k = k_md_products<T, ND>;
+				constexpr int nt = 32 * kPlanes<ND>;
+				k<<<resident_grid(c, k, nt, (n * ring.S + 31) / 32), nt, 0, c.stream>>>(g, ring, x0, n, t0, u, W, A);
+				MESH_LAUNCH_CHECK();
+			};
+			auto force = [&](int x0, int n, RedSlot slot) {
+				auto k = Uout ? k_md_force<T, ND, true> : k_md_force<T, ND, false>;
+				constexpr int nt = 32 * ND;
+				unsigned b = resident_grid(c, k, nt, (n * ring.S + 31) / 32);
+				k<<<b < unsigned(kMaxRedBlocks) ? b : unsigned(kMaxRedBlocks), nt, 0, c.stream>>>(
+				    g, ring, x0, n, u, W, A, p, T(coef), slot, uo, T(tu), reunit ? 1 : 0);
+				MESH_LAUNCH_CHECK();
+			};
+			if (ring.whole)
+			{
+				products(0, g.L[0], 0);
+				force(0, g.L[0], kin ? *kin : RedSlot{});
+				return true;
+			}
+			products(g.L[0] - 1, 1, 0);
+			for (int x0 = 0; x0 < g.L[0]; x0 += ring.R - 1)
+			{
+				int n = g.L[0] - x0 < ring.R - 1 ? g.L[0] - x0 : ring.R - 1;
+				products(x0, n, x0 + 1);
+				force(x0, n, RedSlot{});
+			}
+			if (kin) // a sum over the slabs' launches
+				norm2(P, *kin);
+			return true;
+		}
+		return false;
+	}
 	// ---- fused momentum step + link update (trajectory) ----------------------
 	static constexpr int kMdFirst = 14, kMdLast = 57; // thread-per-site and line-march variants
 	static bool md_supported(Geom const &g)
@@ -2523,8 +2594,10 @@ template <int GRP, class T, int ND> struct Ops
 	// momentum step P -= coef F(Uin) fused with the link update
 	// Uout = exp(tu P) Uin; false (nothing launched) where no fused variant fits
 	static bool hmc_md_step(Field &P, Field const &Uin, Field &Uout, double coef, double tu, bool reunit,
-	                        RedSlot *kin)
+	                        RedSlot *kin, MdScratch const &scratch)
 	{
+		if (products_step(P, Uin, &Uout, coef, tu, reunit, kin, scratch))
+			return true;
 		if (!md_supported(Uin.geom))
 			return false;
 		int v = choose_md(P, Uin, Uout);
@@ -2597,14 +2670,18 @@ template <int GRP, class T, int ND> struct Ops
 		return bestv;
 	}
 	static void tune(Field &P, Field const &U) { choose_force(P, U); }
-	static void momentum_step(Field &P, Field const &U, double coef, RedSlot *kin)
+	static void momentum_step(Field &P, Field const &U, double coef, RedSlot *kin, MdScratch const &scratch)
 	{
+		if (products_step(P, U, nullptr, coef, 0.0, false, kin, scratch))
+			return;
 		int v = choose_force(P, U);
 		launch_force(v, P, U, T(coef), kin ? *kin : RedSlot{});
 	}
 	static void hmc_tune(Field &P, Field const &U) { choose_force(P, U, true); }
-	static void hmc_momentum_step(Field &P, Field const &U, double coef, RedSlot *kin)
+	static void hmc_momentum_step(Field &P, Field const &U, double coef, RedSlot *kin, MdScratch const &scratch)
 	{
+		if (products_step(P, U, nullptr, coef, 0.0, false, kin, scratch))
+			return;
 		int v = choose_force(P, U, true);
 		launch_force(v, P, U, T(coef), kin ? *kin : RedSlot{}, true);
 	}
@@ -2738,7 +2815,7 @@ template <int GRP, class T, int ND> struct Ops
 		                           exp_apply,    axpy_alg,      gauge_transform, tune,
 		                           hmc_plaquette, hmc_evolve,   hmc_momentum_step, hmc_tune,
 		                           hmc_md_step,   hmc_tune_md,  line_extend,    wilson_rt,
-		                           gauge_sweep,   import_direct, export_direct};
+		                           gauge_sweep,   import_direct, export_direct, md_scratch_bytes};
 		return &t;
 	}
 };

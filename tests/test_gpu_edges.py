@@ -56,3 +56,44 @@ def test_plaquette_tiles(ctx, oracle, g, p, dims):
     U64 = links(oracle, g, dims)
     U = mg.GaugeField(ctx, g, p, mg.Grid(dims)).import_(U64.astype(mg.real_dtype(p)))
     assert mg.plaquette(U) == pytest.approx(oracle.plaquette(g, 2, dims, U64), abs=1e-13 if p == 2 else 1e-6)
+
+
+@pytest.mark.parametrize("dims", SHAPES, ids=lambda d: "x".join(map(str, d)))
+def test_fp64_su3_md_step_from_products(ctx, oracle, dims):
+    """momentum step alone and with the link update, for links that are no
+    group elements (the forces are those of the staples for any matrices)"""
+    U64 = links(oracle, 3, dims) * 1.01
+    P64 = oracle.random_momenta(3, 2, dims, 11, 0)
+    U = mg.GaugeField(ctx, 3, 2, mg.Grid(dims)).import_(U64)
+    P = mg.Momenta(ctx, 3, 2, mg.Grid(dims)).import_(P64)
+    mg.momentum_step(P, U, 5.7, 0.3)
+    Po = oracle.momentum_step(3, 2, dims, U64, P64, 5.7, 0.3)
+    assert rel(P.export(), Po) < 1e-12
+    h = mg.Hmc(ctx, 3, 2, mg.Grid(dims), seed=1)
+    h.U.import_(U64)
+    h.P.import_(P64)
+    h.md_step(5.7, 0.3, 0.25)
+    assert rel(h.P.export(), Po) < 1e-12
+    assert rel(h.U.export(), oracle.evolve(3, 2, dims, U64, Po, 0.25)) < 1e-12
+
+
+@pytest.mark.parametrize("dims", [[32, 16, 16, 16], [2, 36, 44, 46], [6, 48, 40, 22]], ids=lambda d: "x".join(map(str, d)))
+def test_fp64_su3_md_step_in_slabs(ctx, dims):
+    """lattices whose products exceed the scratch (slabs of dimension 0; the
+    smallest ring, a ring that does not divide the extent): the same step as the
+    thread-per-link kernel, and the kinetic energy of a whole trajectory"""
+    grid = mg.Grid(dims)
+    out = []
+    for variant in (-1, 0):
+        h = mg.Hmc(ctx, 3, 2, grid, seed=3)
+        h.randomize_gauge_field()
+        P = mg.Momenta(ctx, 3, 2, grid).random(5)
+        try:
+            mg.force_variant(variant)
+            rec = h.update_supplied(P, 0.0, 5.7, [0.05, 0.1, 0.05])
+        finally:
+            mg.force_variant(-1)
+        out.append((rec, h.U.export(), h.P.export()))
+    (ra, ua, pa), (rb, ub, pb) = out
+    assert rel(ua, ub) < 1e-12 and rel(pa, pb) < 1e-12
+    assert ra["H_new"] == pytest.approx(rb["H_new"], rel=1e-12)

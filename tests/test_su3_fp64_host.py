@@ -1,8 +1,8 @@
 """FP64 SU(3) arithmetic of the device code, compiled for the host (it is
 __host__ __device__) and compared with long double: the products as chains of
 fused multiply-adds, their accumulating forms, and the exponential on both
-sides of the norms where its series order changes and where the closed form
-takes over. No GPU needed."""
+sides of the norm where the closed form takes over from the series. No GPU
+needed."""
 import os
 import shutil
 import subprocess
@@ -105,8 +105,8 @@ int main()
 		D::add_mul_adj(r, a, b);
 		e_prod = std::fmax(e_prod, off(r, add(S, adj(mul(A, B)))));
 	}
-	// |X| from far below the first threshold (0.2) past the second (1)
-	double const norms[] = {0, 1e-9, 1e-3, 0.05, 0.1999, 0.2001, 0.5, 0.9999, 1.0001, 2.0};
+	// |X| from zero past the bound of the series (1)
+	double const norms[] = {0, 1e-9, 1e-3, 0.05, 0.1999, 0.2001, 0.4999, 0.5, 0.5001, 0.9999, 1.0001, 2.0};
 	for (double n : norms)
 		for (int t = 0; t < 200; ++t)
 		{
