@@ -257,7 +257,7 @@ bool capturing(Context const &c)
 MdScratch ctx_md_scratch(Field const &U)
 {
 	Context &c = *U.ctx;
-	size_t need = ops_for(U).md_scratch_bytes(U.geom);
+	size_t need = ops_for(U).md_scratch_bytes(U.geom, false);
 	if (need == 0 || capturing(c))
 		return {};
 	if (c.md_bytes < need)
@@ -371,7 +371,7 @@ struct mesh_hmc_s
 	// for it steps without it
 	void ensure_scratch()
 	{
-		size_t need = ops_for(U.f).md_scratch_bytes(U.f.geom);
+		size_t need = ops_for(U.f).md_scratch_bytes(U.f.geom, true);
 		if (need == 0 || scratch.d || capturing(*ctx))
 			return;
 		if (cudaMalloc(&scratch.d, need) == cudaSuccess)
@@ -416,7 +416,8 @@ struct mesh_hmc_s
 			{
 				RedSlot kin = rs(K_NEW);
 				RedSlot *k = i == last_p ? &kin : nullptr;
-				if (i + 1 < n && ops.hmc_md_step(p, *cur, *spare, coef0 * deltas[i], deltas[i + 1], i + 1 == n - 1, k, scratch))
+				if (i + 1 < n && ops.hmc_md_step(p, *cur, *spare, coef0 * deltas[i], deltas[i + 1], i + 1 == n - 1, k, scratch,
+				                                 i + 1 == n - 1))
 				{
 					std::swap(cur, spare);
 					++i; // the link update i + 1 is done
@@ -1197,7 +1198,7 @@ int mesh_hmc_md_step(mesh_hmc h, double beta, double dp, double du)
 		auto const &ops = ops_for(U);
 		h->ensure_scratch();
 		double coef = beta / (2.0 * group_nc(U.group)) * dp;
-		if (ops.hmc_md_step(P, U, h->Ut.f, coef, du, false, nullptr, h->scratch))
+		if (ops.hmc_md_step(P, U, h->Ut.f, coef, du, false, nullptr, h->scratch, true))
 		{
 			// the new links are in Ut: swap the buffers (a captured trajectory
 			// holds the old addresses, so it is dropped)
@@ -1279,13 +1280,8 @@ int mesh_hmc_run(mesh_hmc h, double beta, double const *deltas, int n, int count
 			h->S_valid = true;
 		}
 		h->ensure_scratch();
-		// choose launch variants before capturing (tuning times kernels); the
-		// step from stored products has none
-		if (!h->scratch.d || force_override() >= 0)
-		{
-			ops_for(h->U.f).hmc_tune(h->P.f, h->Unew.f);
-			ops_for(h->U.f).hmc_tune_md(h->P.f, h->Unew.f, h->Ut.f);
-		}
+		// choose launch variants before capturing (tuning times kernels)
+		ops_for(h->U.f).hmc_tune_md(h->P.f, h->Unew.f, h->Ut.f, h->scratch);
 		std::vector<double> dv(deltas, deltas + n);
 		if (!h->graph || h->graph_beta != beta || h->graph_deltas != dv || h->graph_hist != h->d_hist)
 		{

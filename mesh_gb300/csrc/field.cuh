@@ -115,22 +115,20 @@ struct OpsTable
 	void (*exp_apply)(Field &dst, Field const &F, double eps, Field const &g);
 	void (*axpy_alg)(Field &y, double a, Field const &x);
 	void (*gauge_transform)(Field &U, Field const &g);
-	// pick launch variants for U's lattice ahead of a stream capture
-	void (*tune)(Field &P, Field const &U);
 	// the HMC trajectory's plaquette, link update, momentum step and tuning:
 	// links known to be special unitary (SU(3) FP32 links are read as rows 0
 	// and 1, row 2 rebuilt); the same as the generic ones otherwise
 	void (*hmc_plaquette)(Field const &U, RedSlot out);
 	void (*hmc_evolve)(Field const &Usrc, Field &Udst, Field const &P, double t, bool reunit);
 	void (*hmc_momentum_step)(Field &P, Field const &U, double coef, RedSlot *kin, MdScratch const &scratch);
-	void (*hmc_tune)(Field &P, Field const &U);
 	// the trajectory's momentum step fused with the link update after it:
 	// P -= coef F(Uin), Uout = exp(tu P) Uin (reunitised when `reunit`);
 	// returns false, launching nothing, where the fused kernel does not apply
 	// (then the two steps run separately)
+	// without row2 the third rows of FP32 SU(3) links may be left unwritten
 	bool (*hmc_md_step)(Field &P, Field const &Uin, Field &Uout, double coef, double tu, bool reunit, RedSlot *kin,
-	                    MdScratch const &scratch);
-	void (*hmc_tune_md)(Field &P, Field const &Uin, Field &Uout);
+	                    MdScratch const &scratch, bool row2);
+	void (*hmc_tune_md)(Field &P, Field const &Uin, Field &Uout, MdScratch const &scratch);
 	// Wilson loops (4D): Lout = Lprev U_dir(x + (n-1) dir); sum of the r x t loops
 	void (*line_extend)(Field const &U, int dir, int n, void const *Lprev, void *Lout);
 	void (*wilson_rt)(Field const &U, int r, int t, void const *S, void const *Tt, RedSlot out);
@@ -140,7 +138,8 @@ struct OpsTable
 	void (*import_direct)(Field &f, void const *host);
 	void (*export_direct)(Field const &f, void *host);
 	// bytes of scratch the momentum step runs with on this lattice (0: none)
-	size_t (*md_scratch_bytes)(Geom const &g);
+	// with `rows`, of the trajectory's step on special unitary links
+	size_t (*md_scratch_bytes)(Geom const &g, bool rows);
 };
 
 // autotuning registry (tune.cu): variant index per kernel/lattice key

@@ -117,7 +117,7 @@ template <int ND> __device__ __forceinline__ int64_t eo_of_lex(Geom const &g, in
 	for (int i = ND - 1; i >= 0; --i)
 	{
 		uint32_t L = uint32_t(g.L[i]);
-		uint32_t q = uint32_t((uint64_t(r) * g.dm[i]) >> g.ds[i]);
+		uint32_t q = div_extent(g, r, i);
 		sum += int(r - q * L);
 		r = q;
 	}
@@ -1805,6 +1805,7 @@ __global__ void __launch_bounds__(kBlock) k_gauge_transform(Geom g, T *__restric
 } // namespace meshgb
 #include "md_line.cuh"
 #include "md_products.cuh"
+#include "md_plaquettes.cuh"
 namespace meshgb {
 
 // ---------------------------------------------------------------------------
@@ -2404,62 +2405,129 @@ template <int GRP, class T, int ND> struct Ops
 		b = unsigned(ts.ntiles < cap ? ts.ntiles : cap);
 		return ts;
 	}
-	// ---- FP64 SU(3): momentum step from stored products (md_products.cuh) -----
+	// ---- SU(3): the momentum step from stored link products (FP64, any links:
+	// md_products.cuh) or stored plaquettes (FP32 links of the trajectory, special
+	// unitary: md_plaquettes.cuh) -------------------------------------------------
 	static constexpr bool kProducts = GRP == SU3 && sizeof(T) == 8;
-	static size_t md_scratch_bytes(Geom const &g)
+	static constexpr bool kPlaquettes = kRows<GRP, T>;
+	// bytes of scratch a site; rows: links known to be special unitary
+	static size_t md_site_bytes(bool rows)
 	{
-		size_t bytes = 0;
 		if constexpr (kProducts)
-			md_ring<T, ND>(g, &bytes);
+			return sizeof(T) * (2 * kPlanes<ND> * Gp::NR + kPlanes<ND> * Gp::NA);
+		return kPlaquettes && rows ? sizeof(T) * kPlanes<ND> * Gp::NA : 0;
+	}
+	static size_t md_scratch_bytes(Geom const &g, bool rows)
+	{
+		size_t bytes = 0, site = md_site_bytes(rows);
+		if (kPlaquettes && !LinkLoadSU3R32::fits(g.V))
+			site = 0; // 32-bit offsets
+		if (site)
+			md_ring(g, site, &bytes);
 		return bytes;
 	}
+	// walks the lattice: first(x0, n, t0) fills the ring, second(x0, n) uses it
+	template <class A, class B> static void md_slabs(Geom const &g, MdRing const &ring, A &&first, B &&second)
+	{
+		if (ring.whole)
+		{
+			first(0, g.L[0], 0);
+			second(0, g.L[0]);
+			return;
+		}
+		first(g.L[0] - 1, 1, 0);
+		for (int x0 = 0; x0 < g.L[0]; x0 += ring.R - 1)
+		{
+			int n = g.L[0] - x0 < ring.R - 1 ? g.L[0] - x0 : ring.R - 1;
+			first(x0, n, x0 + 1);
+			second(x0, n);
+		}
+	}
 	// false (nothing launched) without scratch or with a pinned launch variant
-	static bool products_step(Field &P, Field const &U, Field *Uout, double coef, double tu, bool reunit, RedSlot *kin,
-	                          MdScratch const &scratch)
+	static bool scratch_step(Field &P, Field const &U, Field *Uout, double coef, double tu, bool reunit, RedSlot *kin,
+	                         MdScratch const &scratch, bool rows, bool row2 = true)
+	{
+		Geom const &g = U.geom;
+		size_t bytes = md_scratch_bytes(g, rows);
+		if (!bytes || scratch.bytes < bytes)
+			return false;
+		MdRing ring = md_ring(g, md_site_bytes(rows), &bytes);
+		// a sum over several launches: after them, from P
+		RedSlot slot = kin && ring.whole ? *kin : RedSlot{};
+		if constexpr (kProducts)
+			products_step(P, U, Uout, coef, tu, reunit, slot, ring, scratch);
+		else if constexpr (kPlaquettes)
+		{
+			if (ring.whole)
+				plaquettes_step<true>(P, U, Uout, coef, tu, reunit, slot, ring, scratch, row2);
+			else
+				plaquettes_step<false>(P, U, Uout, coef, tu, reunit, slot, ring, scratch, row2);
+		}
+		if (kin && !ring.whole)
+			norm2(P, *kin);
+		return true;
+	}
+	// grid over the 32-site tiles of n slices, walked by at most the resident
+	// blocks (and the reduction's partial sums)
+	template <class K> static unsigned slab_grid(Context const &c, K kernel, int threads, MdRing const &ring, int n)
+	{
+		unsigned b = resident_grid(c, kernel, threads, slab_tiles(ring.S, n));
+		return b < unsigned(kMaxRedBlocks) ? b : unsigned(kMaxRedBlocks);
+	}
+	static void products_step(Field &P, Field const &U, Field *Uout, double coef, double tu, bool reunit,
+	                          RedSlot const &kin, MdRing const &ring, MdScratch const &scratch)
 	{
 		if constexpr (kProducts)
 		{
-			Geom const &g = U.geom;
-			size_t bytes = 0;
-			MdRing ring = md_ring<T, ND>(g, &bytes);
-			if (!scratch.d || scratch.bytes < bytes || force_override() >= 0)
-				return false;
 			auto &c = *U.ctx;
+			Geom const &g = U.geom;
 			T *W = static_cast<T *>(scratch.d), *A = W + 2 * kPlanes<ND> * Gp::NR * ring.V;
 			T const *u = static_cast<T const *>(U.d);
 			T *p = static_cast<T *>(P.d), *uo = Uout ? static_cast<T *>(Uout->d) : nullptr;
-			auto products = [&](int x0, int n, int t0) {
-				auto k = k_md_products<T, ND>;
-				constexpr int nt = 32 * kPlanes<ND>;
-				k<<<resident_grid(c, k, nt, (n * ring.S + 31) / 32), nt, 0, c.stream>>>(g, ring, x0, n, t0, u, W, A);
-				MESH_LAUNCH_CHECK();
-			};
-			auto force = [&](int x0, int n, RedSlot slot) {
-				auto k = Uout ? k_md_force<T, ND, true> : k_md_force<T, ND, false>;
-				constexpr int nt = 32 * ND;
-				unsigned b = resident_grid(c, k, nt, (n * ring.S + 31) / 32);
-				k<<<b < unsigned(kMaxRedBlocks) ? b : unsigned(kMaxRedBlocks), nt, 0, c.stream>>>(
-				    g, ring, x0, n, u, W, A, p, T(coef), slot, uo, T(tu), reunit ? 1 : 0);
-				MESH_LAUNCH_CHECK();
-			};
-			if (ring.whole)
-			{
-				products(0, g.L[0], 0);
-				force(0, g.L[0], kin ? *kin : RedSlot{});
-				return true;
-			}
-			products(g.L[0] - 1, 1, 0);
-			for (int x0 = 0; x0 < g.L[0]; x0 += ring.R - 1)
-			{
-				int n = g.L[0] - x0 < ring.R - 1 ? g.L[0] - x0 : ring.R - 1;
-				products(x0, n, x0 + 1);
-				force(x0, n, RedSlot{});
-			}
-			if (kin) // a sum over the slabs' launches
-				norm2(P, *kin);
-			return true;
+			md_slabs(
+			    g, ring,
+			    [&](int x0, int n, int t0) {
+				    auto k = k_md_products<T, ND>;
+				    constexpr int nt = 32 * kPlanes<ND>;
+				    k<<<slab_grid(c, k, nt, ring, n), nt, 0, c.stream>>>(g, ring, x0, n, t0, u, W, A);
+				    MESH_LAUNCH_CHECK();
+			    },
+			    [&](int x0, int n) {
+				    auto k = Uout ? k_md_force<T, ND, true> : k_md_force<T, ND, false>;
+				    constexpr int nt = 32 * ND;
+				    k<<<slab_grid(c, k, nt, ring, n), nt, 0, c.stream>>>(g, ring, x0, n, u, W, A, p, T(coef), kin, uo, T(tu),
+				                                                        reunit ? 1 : 0);
+				    MESH_LAUNCH_CHECK();
+			    });
 		}
-		return false;
+	}
+	template <bool WHOLE>
+	static void plaquettes_step(Field &P, Field const &U, Field *Uout, double coef, double tu, bool reunit,
+	                            RedSlot const &kin, MdRing const &ring, MdScratch const &scratch, bool row2)
+	{
+		if constexpr (kPlaquettes)
+		{
+			auto &c = *U.ctx;
+			Geom const &g = U.geom;
+			LinkLoadSU3R32 ld{static_cast<float4 const *>(U.d), uint32_t(g.V), uint32_t(g.V / 2 * 9)};
+			AlgR32 A{static_cast<float4 *>(scratch.d), uint32_t(ring.V)};
+			T *p = static_cast<T *>(P.d), *uo = Uout ? static_cast<T *>(Uout->d) : nullptr;
+			md_slabs(
+			    g, ring,
+			    [&](int x0, int n, int t0) {
+				    auto k = k_md_plaquettes<ND, WHOLE>;
+				    constexpr int nt = 32 * kPlanes<ND>;
+				    k<<<slab_grid(c, k, nt, ring, n), nt, 0, c.stream>>>(g, ring, x0, n, t0, ld, A);
+				    MESH_LAUNCH_CHECK();
+			    },
+			    [&](int x0, int n) {
+				    auto k = Uout ? k_md_transport<ND, true, WHOLE> : k_md_transport<ND, false, WHOLE>;
+				    constexpr int nt = 32 * ND;
+				    k<<<slab_grid(c, k, nt, ring, n), nt, 0, c.stream>>>(g, ring, x0, n, ld, A, p, T(coef), kin, uo, T(tu),
+				                                                        reunit ? 1 : 0, row2 ? 1 : 0);
+				    MESH_LAUNCH_CHECK();
+			    });
+		}
 	}
 	// ---- fused momentum step + link update (trajectory) ----------------------
 	static constexpr int kMdFirst = 14, kMdLast = 57; // thread-per-site and line-march variants
@@ -2511,8 +2579,14 @@ template <int GRP, class T, int ND> struct Ops
 	// once with coef = 0 and tu = 0 (P unchanged, Uout = Uin); not while the
 	// stream is capturing
 	static constexpr int kSeparate = 1000; // the two steps as separate kernels were faster
-	static int choose_md(Field &P, Field const &Uin, Field &Uout)
+	static constexpr int kStored = 1001;   // the step from stored plaquettes was faster
+	static bool stored_applies(Geom const &g, MdScratch const &scratch)
 	{
+		return kPlaquettes && scratch.bytes >= md_scratch_bytes(g, true) && md_scratch_bytes(g, true) > 0;
+	}
+	static int choose_md(Field &P, Field const &Uin, Field &Uout, MdScratch const &scratch)
+	{
+		bool stored = stored_applies(Uin.geom, scratch);
 		int ov = force_override();
 		if (ov >= kMdFirst && ov <= kMdLast && force_variant_valid(Uin.geom, ov))
 			return ov;
@@ -2521,13 +2595,15 @@ template <int GRP, class T, int ND> struct Ops
 		std::string key = "md_step/group" + std::to_string(GRP) + "/" + (sizeof(T) == 4 ? "f32" : "f64") + "/";
 		for (int i = 0; i < ND; ++i)
 			key += (i ? "x" : "") + std::to_string(Uin.dims[i]);
-		int v = tuned_variant(key);
-		if (v >= 0)
-			return v;
-		int dflt = -1;
-		for (int cand = kMdFirst; cand <= kMdLast && dflt < 0; ++cand)
+		// where nothing is timed, and for a chain without the scratch that the
+		// lattice was tuned with
+		int dflt = stored ? kStored : kSeparate;
+		for (int cand = kMdFirst; cand <= kMdLast && dflt == kSeparate; ++cand)
 			if (force_variant_valid(Uin.geom, cand))
 				dflt = cand;
+		int v = tuned_variant(key);
+		if (v >= 0)
+			return v == kStored && !stored ? dflt : v;
 		cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
 		cudaStreamIsCapturing(Uin.ctx->stream, &cs);
 		if (cs != cudaStreamCaptureStatusNone || !autotune_enabled())
@@ -2576,7 +2652,7 @@ template <int GRP, class T, int ND> struct Ops
 			float ms = 0;
 			MESH_CUDA(cudaEventElapsedTime(&ms, e0, e1));
 			ms /= 3;
-			report += std::string(", separate ") + force_variant(fv).name + " + link update=" +
+			report += std::string(report.empty() ? "separate " : ", separate ") + force_variant(fv).name + " + link update=" +
 			          std::to_string(ms * 1000.0f) + "us";
 			if (ms < best)
 			{
@@ -2584,32 +2660,61 @@ template <int GRP, class T, int ND> struct Ops
 				bestv = kSeparate;
 			}
 		}
+		if (stored)
+		{
+			auto step = [&] { scratch_step(P, Uin, &Uout, 0.0, 0.0, false, nullptr, scratch, true, true); };
+			step();
+			MESH_CUDA(cudaEventRecord(e0, c.stream));
+			for (int r = 0; r < 3; ++r)
+				step();
+			MESH_CUDA(cudaEventRecord(e1, c.stream));
+			MESH_CUDA(cudaEventSynchronize(e1));
+			float ms = 0;
+			MESH_CUDA(cudaEventElapsedTime(&ms, e0, e1));
+			ms /= 3;
+			report += ", stored plaquettes=" + std::to_string(ms * 1000.0f) + "us";
+			if (ms < best)
+			{
+				best = ms;
+				bestv = kStored;
+			}
+		}
 		cudaEventDestroy(e0);
 		cudaEventDestroy(e1);
 		set_tuned_variant(key, bestv,
-		                  std::string("chosen ") + (bestv == kSeparate ? "separate kernels" : force_variant(bestv).name) +
+		                  std::string("chosen ") +
+		                      (bestv == kSeparate ? "separate kernels"
+		                       : bestv == kStored ? "stored plaquettes"
+		                                          : force_variant(bestv).name) +
 		                      " [" + report + "]");
 		return bestv;
 	}
 	// momentum step P -= coef F(Uin) fused with the link update
 	// Uout = exp(tu P) Uin; false (nothing launched) where no fused variant fits
 	static bool hmc_md_step(Field &P, Field const &Uin, Field &Uout, double coef, double tu, bool reunit,
-	                        RedSlot *kin, MdScratch const &scratch)
+	                        RedSlot *kin, MdScratch const &scratch, bool row2)
 	{
-		if (products_step(P, Uin, &Uout, coef, tu, reunit, kin, scratch))
+		if (kProducts && force_override() < 0 && scratch_step(P, Uin, &Uout, coef, tu, reunit, kin, scratch, true))
 			return true;
-		if (!md_supported(Uin.geom))
+		if (!md_supported(Uin.geom) && !stored_applies(Uin.geom, scratch))
 			return false;
-		int v = choose_md(P, Uin, Uout);
+		int v = choose_md(P, Uin, Uout, scratch);
 		if (v == kSeparate)
 			return false;
+		if (v == kStored)
+			return scratch_step(P, Uin, &Uout, coef, tu, reunit, kin, scratch, true, row2);
 		launch_md(v, P, Uin, Uout, T(coef), T(tu), reunit ? 1 : 0, kin ? *kin : RedSlot{});
 		return true;
 	}
-	static void hmc_tune_md(Field &P, Field const &Uin, Field &Uout)
+	// the launch variants of a trajectory's steps (timed outside a capture); the
+	// step from stored products has none
+	static void hmc_tune_md(Field &P, Field const &Uin, Field &Uout, MdScratch const &scratch)
 	{
-		if (md_supported(Uin.geom))
-			choose_md(P, Uin, Uout);
+		if (kProducts && force_override() < 0 && scratch.bytes >= md_scratch_bytes(Uin.geom, true))
+			return;
+		choose_force(P, Uin, true);
+		if (md_supported(Uin.geom) || stored_applies(Uin.geom, scratch))
+			choose_md(P, Uin, Uout, scratch);
 	}
 	static std::string force_key(Field const &U, bool rows)
 	{
@@ -2669,18 +2774,16 @@ template <int GRP, class T, int ND> struct Ops
 		set_tuned_variant(key, bestv, std::string("chosen ") + force_variant(bestv).name + " [" + report + "]");
 		return bestv;
 	}
-	static void tune(Field &P, Field const &U) { choose_force(P, U); }
 	static void momentum_step(Field &P, Field const &U, double coef, RedSlot *kin, MdScratch const &scratch)
 	{
-		if (products_step(P, U, nullptr, coef, 0.0, false, kin, scratch))
+		if (kProducts && force_override() < 0 && scratch_step(P, U, nullptr, coef, 0.0, false, kin, scratch, false))
 			return;
 		int v = choose_force(P, U);
 		launch_force(v, P, U, T(coef), kin ? *kin : RedSlot{});
 	}
-	static void hmc_tune(Field &P, Field const &U) { choose_force(P, U, true); }
 	static void hmc_momentum_step(Field &P, Field const &U, double coef, RedSlot *kin, MdScratch const &scratch)
 	{
-		if (products_step(P, U, nullptr, coef, 0.0, false, kin, scratch))
+		if (kProducts && force_override() < 0 && scratch_step(P, U, nullptr, coef, 0.0, false, kin, scratch, true))
 			return;
 		int v = choose_force(P, U, true);
 		launch_force(v, P, U, T(coef), kin ? *kin : RedSlot{}, true);
@@ -2812,8 +2915,8 @@ template <int GRP, class T, int ND> struct Ops
 		                           cshift,       site_op,       sum_real_trace, plaquette,      staple_sum,
 		                           wilson_deriv, reunitize,     evolve,         momentum_step,  landau_functional,
 		                           landau_theta, landau_deriv,  landau_or_half, reunit_exact,   alg_dot,
-		                           exp_apply,    axpy_alg,      gauge_transform, tune,
-		                           hmc_plaquette, hmc_evolve,   hmc_momentum_step, hmc_tune,
+		                           exp_apply,    axpy_alg,      gauge_transform,
+		                           hmc_plaquette, hmc_evolve,   hmc_momentum_step,
 		                           hmc_md_step,   hmc_tune_md,  line_extend,    wilson_rt,
 		                           gauge_sweep,   import_direct, export_direct, md_scratch_bytes};
 		return &t;

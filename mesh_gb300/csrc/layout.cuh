@@ -31,10 +31,12 @@ struct Geom
 	int L[4];
 	int64_t V, Vh;
 	int64_t stride[4]; // lexicographic stride of dimension i
-	// division by L[i] as a multiply and shift: n / L[i] == (n * dm[i]) >> ds[i]
-	// for every n < 2^31 (ds = 31 + ceil(log2 L), dm = floor(2^ds / L) + 1 <
-	// 2^33, so n * dm < 2^64; the rounding error n / 2^ds < 1 / L)
-	uint64_t dm[4];
+	// division by L[i] as a multiply and shift: n / L[i] == (n * dm[i] >> 32) >>
+	// ds[i] for every n < 2^31 and L >= 2 (l = ceil(log2 L), ds = l - 1, dm =
+	// floor(2^(31 + l) / L) + 1 < 2^32 as 2^l < 2 L; the rounding error n /
+	// 2^(31 + l) < 1 / L). One wide multiply and a shift; with 64-bit factors it
+	// was four times the instructions, in every kernel that starts from a site
+	uint32_t dm[4];
 	int ds[4];
 
 	// extent / stride of a runtime direction through selects on constant
@@ -69,11 +71,23 @@ inline Geom make_geom(int nd, int32_t const *dims)
 		int l = 0;
 		while ((1 << l) < g.L[i])
 			++l;
-		g.ds[i] = 31 + l;
-		g.dm[i] = (uint64_t(1) << g.ds[i]) / uint64_t(g.L[i]) + 1;
+		if (l == 0) // a dimension that is not there
+			continue;
+		g.ds[i] = l - 1;
+		g.dm[i] = uint32_t((uint64_t(1) << (31 + l)) / uint64_t(g.L[i]) + 1);
 	}
 	g.Vh = g.V / 2;
 	return g;
+}
+
+// r / L[i] for r < 2^31
+__host__ __device__ __forceinline__ uint32_t div_extent(Geom const &g, uint32_t r, int i)
+{
+#ifdef __CUDA_ARCH__
+	return __umulhi(r, g.dm[i]) >> g.ds[i];
+#else
+	return uint32_t((uint64_t(r) * g.dm[i]) >> 32) >> g.ds[i];
+#endif
 }
 
 // Coordinates, lexicographic index and parity of a site. The coordinates are
@@ -99,7 +113,7 @@ template <int ND> __device__ __forceinline__ Site<ND> site_from_eo(Geom const &g
 	for (int i = ND - 1; i >= 0; --i)
 	{
 		uint32_t L = uint32_t(g.L[i]);
-		uint32_t q = uint32_t((uint64_t(r) * g.dm[i]) >> g.ds[i]);
+		uint32_t q = div_extent(g, r, i);
 		uint32_t xi = r - q * L;
 		px |= xi << (8 * i);
 		r = q;

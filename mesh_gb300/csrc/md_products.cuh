@@ -48,11 +48,16 @@ __device__ __forceinline__ int64_t ring_index(MdRing const &r, int32_t lex, int 
 	return int64_t(par) * (r.V / 2) + (l >> 1);
 }
 
-// site i (0 <= i < n S) of the slices [x0, x0 + n): even sites first
-__device__ __forceinline__ int64_t slab_site(Geom const &g, int64_t S, int x0, int64_t half, int64_t i)
+// tiles of 32 sites of n slices; tile 2j holds the j-th 32 even sites, 2j + 1 the
+// odd ones beside them (all even sites first read every neighbour link, of odd
+// sites, long before the odd sites did: twice the DRAM traffic)
+__host__ __device__ __forceinline__ int slab_tiles(int64_t S, int n) { return 2 * int((n * (S / 2) + 31) / 32); }
+// this lane's site of a tile of the slices [x0, x0 + n), false past the end
+__device__ __forceinline__ bool slab_site(Geom const &g, int64_t S, int x0, int n, int tile, int64_t &s)
 {
-	int p = i >= half;
-	return (p ? g.Vh - half : 0) + int64_t(x0) * (S / 2) + i;
+	int32_t j = (tile >> 1) * 32 + int32_t(threadIdx.x & 31), h = int32_t(S / 2);
+	s = int64_t(tile & 1) * g.Vh + int64_t(x0) * h + j;
+	return j < n * h;
 }
 
 // products of the slices [x0, x0 + n) into the ring, slice x0 at t = t0
@@ -64,10 +69,12 @@ __global__ void __launch_bounds__(32 * kPlanes<ND>)
 	using E = typename Gp::E;
 	LinkLoad<SU3, T, ND> ld{U, g.V};
 	int q = threadIdx.x >> 5, mu = plane_mu<ND>(q), nu = plane_nu<ND>(q);
-	int64_t sites = n * ring.S;
-	for (int64_t i = int64_t(blockIdx.x) * 32 + (threadIdx.x & 31); i < sites; i += int64_t(gridDim.x) * 32)
+	int ntiles = slab_tiles(ring.S, n);
+	for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x)
 	{
-		int64_t s = slab_site(g, ring.S, x0, sites / 2, i);
+		int64_t s;
+		if (!slab_site(g, ring.S, x0, n, tile, s))
+			continue;
 		Site<ND> st = site_from_eo<ND>(g, s);
 		int64_t k = ring_index(ring, st.lex, st.x(0), t0 + st.x(0) - x0, st.par);
 		E ab = Gp::mul(ld(mu, s), ld(nu, eo_shift1<ND>(g, st, mu, +1)));
@@ -93,11 +100,13 @@ __global__ void __launch_bounds__(32 * ND)
 	using E = typename Gp::E;
 	LinkLoad<SU3, T, ND> ld{U, g.V};
 	int mu = threadIdx.x >> 5;
-	int64_t sites = n * ring.S;
+	int ntiles = slab_tiles(ring.S, n);
 	double acc = 0.0;
-	for (int64_t i = int64_t(blockIdx.x) * 32 + (threadIdx.x & 31); i < sites; i += int64_t(gridDim.x) * 32)
+	for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x)
 	{
-		int64_t s = slab_site(g, ring.S, x0, sites / 2, i);
+		int64_t s;
+		if (!slab_site(g, ring.S, x0, n, tile, s))
+			continue;
 		Site<ND> st = site_from_eo<ND>(g, s);
 		int64_t k = ring_index(ring, st.lex, st.x(0), st.x(0) + 1, st.par);
 		T f[Gp::NA];
@@ -153,13 +162,12 @@ __global__ void __launch_bounds__(32 * ND)
 		grid_sum<32 * ND>(acc, kin);
 }
 
-// the ring of a lattice within the cap, and its bytes
-template <class T, int ND> inline MdRing md_ring(Geom const &g, size_t *bytes)
+// the ring of a lattice within the cap (site_bytes held for a site), and its bytes
+inline MdRing md_ring(Geom const &g, size_t site_bytes, size_t *bytes)
 {
-	constexpr int kReals = 2 * kPlanes<ND> * Group<SU3, T>::NR + kPlanes<ND> * Group<SU3, T>::NA;
 	MdRing r{};
 	r.S = g.V / g.L[0];
-	size_t slice = size_t(r.S) * kReals * sizeof(T);
+	size_t slice = size_t(r.S) * site_bytes;
 	int64_t fit = int64_t(kMdScratchCap / slice);
 	r.whole = fit >= g.L[0];
 	r.R = r.whole ? g.L[0] : int(fit < 2 ? 2 : fit);

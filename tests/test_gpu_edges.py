@@ -97,3 +97,46 @@ def test_fp64_su3_md_step_in_slabs(ctx, dims):
     (ra, ua, pa), (rb, ub, pb) = out
     assert rel(ua, ub) < 1e-12 and rel(pa, pb) < 1e-12
     assert ra["H_new"] == pytest.approx(rb["H_new"], rel=1e-12)
+
+
+@pytest.mark.parametrize("dims", SHAPES + [[4, 6, 10, 14]], ids=lambda d: "x".join(map(str, d)))
+def test_fp32_su3_step_from_plaquettes(ctx, oracle, dims):
+    """one MD step and a trajectory (whose inner steps write rows 0 and 1 of the
+    links only) of the autotuned chain against the FP64 oracle; small lattices
+    choose the step from stored plaquettes"""
+    U64 = oracle.hmc_chain(3, 2, dims, oracle.unit_gauge(3, 2, dims), 5.7, oracle.make_deltas("2lf", 0.5, 8), 3, 0, 2)[0]
+    P64 = oracle.random_momenta(3, 2, dims, 11, 0)
+    U32, P32 = U64.astype(np.float32), P64.astype(np.float32)
+    h = mg.Hmc(ctx, 3, mg.F32, mg.Grid(dims), seed=1)
+    h.U.import_(U32)
+    h.P.import_(P32)
+    h.md_step(5.7, 0.07, 0.05)
+    Po = oracle.momentum_step(3, 2, dims, U64, P64, 5.7, 0.07)
+    assert rel(h.P.export(), Po) < 2e-5
+    assert rel(h.U.export(), oracle.evolve(3, 2, dims, U64, Po, 0.05)) < 2e-5
+    h.U.import_(U32)
+    d = oracle.make_deltas("2mn", 0.5, 5)
+    h.update_supplied(mg.Momenta(ctx, 3, mg.F32, mg.Grid(dims)).import_(P32), 0.0, 5.7, d)
+    U_new, _ = oracle.hmc_update(3, 2, dims, U64, P64, 5.7, d, 0.0)
+    assert rel(h.U.export(), U_new) < 2e-5
+
+
+def test_fp32_su3_step_from_plaquettes_in_slabs(ctx):
+    """a lattice whose plaquettes exceed the scratch: the trajectory of the
+    thread-per-link kernel"""
+    dims = [40, 32, 34, 32]
+    out = []
+    for variant in (-1, 0):
+        h = mg.Hmc(ctx, 3, mg.F32, mg.Grid(dims), seed=3)
+        h.U.random(9)
+        P = mg.Momenta(ctx, 3, mg.F32, mg.Grid(dims)).random(5)
+        try:
+            mg.force_variant(variant)
+            rec = h.update_supplied(P, 0.0, 5.7, [0.05, 0.1, 0.05, 0.1, 0.05])
+        finally:
+            mg.force_variant(-1)
+        out.append((rec, h.U.export(), h.P.export()))
+    (ra, ua, pa), (rb, ub, pb) = out
+    assert "stored plaquettes" in [ln for ln in mg.tune_report().splitlines() if "md_step/group3/f32/40x32x34x32" in ln][0]
+    assert rel(ua, ub) < 2e-5 and rel(pa, pb) < 2e-5
+    assert ra["H_new"] == pytest.approx(rb["H_new"], rel=1e-6)
