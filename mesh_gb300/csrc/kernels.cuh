@@ -1237,8 +1237,14 @@ __global__ void __launch_bounds__(NT, MINB)
 // parity do not enter each other's staples (those read U_mu only at x +- nu,
 // of the other parity), so they are updated together
 // ---------------------------------------------------------------------------
+// blocks of 64 under 128 registers, eight per SM: unbounded, the kernel took 130
+// registers and one block of 256 filled an SM (8 warps, 40% of the issue slots).
+// SU(3) FP32 on a GB300, half a direction of overrelaxation / heat-bath: 32^4 122 /
+// 231 -> 87 / 180 us, 12x20x14x30 16.7 / 34 -> 12.6 / 25 us; more warps under fewer
+// registers spill (102 us at 10 blocks, 121 at 12)
+constexpr int kGaugeBlock = 64;
 template <int GRP, class T, int ND, bool OR>
-__global__ void __launch_bounds__(kBlock)
+__global__ void __launch_bounds__(kGaugeBlock, sizeof(T) == 8 ? 4 : 8)
     k_gauge_update(Geom g, int mu, int parity, T *U, double beta, uint64_t seed, uint64_t ctr)
 {
 	using Gp = Group<GRP, T>;
@@ -2879,12 +2885,16 @@ template <int GRP, class T, int ND> struct Ops
 						    <<<resident_grid(c, k_gauge_update_planes<GRP, T, ND, false>, kThreads, nt), kThreads, 0,
 						       c.stream>>>(U.geom, nt, mu, par, u, beta, seed, ctr);
 				}
-				else if (overrelax)
-					k_gauge_update<GRP, T, ND, true>
-					    <<<blocks(c, U.geom.Vh), kBlock, 0, c.stream>>>(U.geom, mu, par, u, beta, seed, ctr);
 				else
-					k_gauge_update<GRP, T, ND, false>
-					    <<<blocks(c, U.geom.Vh), kBlock, 0, c.stream>>>(U.geom, mu, par, u, beta, seed, ctr);
+				{
+					unsigned b = grid_for(c, U.geom.Vh, kGaugeBlock, 64);
+					if (overrelax)
+						k_gauge_update<GRP, T, ND, true>
+						    <<<b, kGaugeBlock, 0, c.stream>>>(U.geom, mu, par, u, beta, seed, ctr);
+					else
+						k_gauge_update<GRP, T, ND, false>
+						    <<<b, kGaugeBlock, 0, c.stream>>>(U.geom, mu, par, u, beta, seed, ctr);
+				}
 				MESH_LAUNCH_CHECK();
 			}
 	}
