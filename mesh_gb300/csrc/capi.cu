@@ -40,8 +40,8 @@ void teardown_ctx(Context &c)
 	cudaFree(c.d_err);
 	if (c.d_stage)
 		cudaFree(c.d_stage);
-	if (c.d_md)
-		cudaFree(c.d_md);
+	if (c.d_work)
+		cudaFree(c.d_work);
 	if (c.own_stream && c.stream)
 		cudaStreamDestroy(c.stream);
 }
@@ -251,30 +251,42 @@ bool capturing(Context const &c)
 	return cudaStreamIsCapturing(c.stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone;
 }
 
-// the context's momentum-step scratch for U's lattice. Empty (the step then
-// runs without it) while the stream is being captured, as a later lattice may
-// replace the memory a captured launch points to, and when there is no memory.
+// The context's workspace for the duration of a call: kept between calls up to
+// Context::kWorkCap, allocated and freed by the call beyond it.
+struct Workspace
+{
+	Context &c;
+	void *d = nullptr;
+	bool own = false;
+	Workspace(Context &ctx, size_t bytes) : c(ctx)
+	{
+		if (bytes <= Context::kWorkCap && !capturing(c) && c.grow_work(bytes))
+			d = c.d_work;
+		else
+		{
+			MESH_CUDA(cudaMallocAsync(&d, bytes, c.stream));
+			own = true;
+		}
+	}
+	~Workspace()
+	{
+		if (own)
+			cudaFreeAsync(d, c.stream);
+	}
+	Workspace(Workspace const &) = delete;
+	Workspace &operator=(Workspace const &) = delete;
+};
+
+// scratch for the momentum step on U's lattice from the context's workspace. Empty
+// (the step then runs without it) while the stream is being captured, as a later
+// call may replace the memory a captured launch points to, and without memory.
 MdScratch ctx_md_scratch(Field const &U)
 {
 	Context &c = *U.ctx;
 	size_t need = ops_for(U).md_scratch_bytes(U.geom, false);
-	if (need == 0 || capturing(c))
+	if (need == 0 || capturing(c) || !c.grow_work(need))
 		return {};
-	if (c.md_bytes < need)
-	{
-		MESH_CUDA(cudaStreamSynchronize(c.stream));
-		cudaFree(c.d_md);
-		c.d_md = nullptr;
-		c.md_bytes = 0;
-		if (cudaMalloc(&c.d_md, need) != cudaSuccess)
-		{
-			cudaGetLastError();
-			c.d_md = nullptr;
-			return {};
-		}
-		c.md_bytes = need;
-	}
-	return {c.d_md, c.md_bytes};
+	return {c.d_work, c.work_bytes};
 }
 
 void check_deltas(double const *deltas, int n)
@@ -488,8 +500,8 @@ int mesh_ctx_create(int device, void *stream, mesh_ctx *out)
 		}
 		MESH_CUDA(cudaMalloc(&c.d_partials, sizeof(double) * size_t(kSlots) * kMaxRedBlocks));
 		MESH_CUDA(cudaMalloc(&c.d_results, sizeof(double) * kSlots));
-		MESH_CUDA(cudaMalloc(&c.d_counters, sizeof(unsigned) * kSlots));
-		MESH_CUDA(cudaMemset(c.d_counters, 0, sizeof(unsigned) * kSlots));
+		MESH_CUDA(cudaMalloc(&c.d_counters, sizeof(unsigned) * kCounters));
+		MESH_CUDA(cudaMemset(c.d_counters, 0, sizeof(unsigned) * kCounters));
 		MESH_CUDA(cudaMemset(c.d_results, 0, sizeof(double) * kSlots));
 		MESH_CUDA(cudaMalloc(&c.d_err, sizeof(int)));
 		MESH_CUDA(cudaMemset(c.d_err, 0, sizeof(int)));
@@ -892,41 +904,21 @@ int mesh_wilson_loops(mesh_field Uh, int max_r, int max_t, double *out)
 		auto const &ops = ops_for(U);
 		size_t comp = size_t(U.geom.V) * size_t(U.nr) * U.real_bytes;
 		size_t nres = size_t(max_r) * size_t(max_t);
-		char *lines = nullptr; // max_t temporal lines, then the three spatial lines
-		double *res = nullptr;
-		MESH_CUDA(cudaMallocAsync(&lines, comp * size_t(max_t + 3), c.stream));
-		MESH_CUDA(cudaMallocAsync(&res, nres * sizeof(double), c.stream));
-		auto release = [&] {
-			cudaFreeAsync(lines, c.stream);
-			cudaFreeAsync(res, c.stream);
-		};
-		try
+		// max_t temporal lines, the three spatial lines, the sums' scratch and results
+		size_t npart = ops.wilson_partials(c, max_t);
+		size_t bytes = comp * size_t(max_t + 3) + (npart + nres) * sizeof(double);
+		Workspace ws(c, bytes);
+		char *T1 = static_cast<char *>(ws.d), *S = T1 + comp * size_t(max_t);
+		double *part = reinterpret_cast<double *>(S + 3 * comp), *res = part + npart;
+		ops.temporal_lines(U, max_t, T1);
+		for (int r = 1; r <= max_r; ++r)
 		{
-			char *T1 = lines, *S = lines + comp * size_t(max_t);
-			char const *u = static_cast<char const *>(U.d);
-			MESH_CUDA(cudaMemcpyAsync(T1, u + 3 * comp, comp, cudaMemcpyDeviceToDevice, c.stream));
-			for (int t = 2; t <= max_t; ++t)
-				ops.line_extend(U, 3, t, T1 + comp * size_t(t - 2), T1 + comp * size_t(t - 1));
-			MESH_CUDA(cudaMemcpyAsync(S, u, 3 * comp, cudaMemcpyDeviceToDevice, c.stream));
-			RedSlot base = slot(c, SLOT_TMP);
-			for (int r = 1; r <= max_r; ++r)
-			{
-				if (r > 1)
-					for (int mu = 0; mu < 3; ++mu)
-						ops.line_extend(U, mu, r, S + comp * mu, S + comp * mu);
-				for (int t = 1; t <= max_t; ++t)
-					ops.wilson_rt(U, r, t, S, T1 + comp * size_t(t - 1),
-					              RedSlot{base.partials, res + size_t(r - 1) * max_t + (t - 1), base.counter});
-			}
-			MESH_CUDA(cudaMemcpyAsync(out, res, nres * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
-			MESH_CUDA(cudaStreamSynchronize(c.stream));
+			ops.spatial_lines(U, r, S);
+			static_assert(256 / 4 <= kCounters - kSlots, "a counter per chunk of extents");
+			ops.wilson_t(U, r, max_t, S, T1, part, c.d_counters + kSlots, res + size_t(r - 1) * max_t);
 		}
-		catch (...)
-		{
-			release();
-			throw;
-		}
-		release();
+		MESH_CUDA(cudaMemcpyAsync(out, res, nres * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
+		MESH_CUDA(cudaStreamSynchronize(c.stream));
 		double norm = 3.0 * double(U.geom.V) * double(group_nc(U.group));
 		for (size_t k = 0; k < nres; ++k)
 			out[k] /= norm;

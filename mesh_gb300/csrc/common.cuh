@@ -39,6 +39,8 @@ inline void require(bool ok, char const *msg, int code = MESH_ERR_ARG)
 // scalars of one HMC trajectory (S_old, S_new, K_old, K_new, ...) and by the
 // synchronous one-off reductions.
 constexpr int kSlots = 64;
+// Last-block counters: one per slot, then those of launches with several sums.
+constexpr int kCounters = 2 * kSlots;
 // Maximum number of blocks of one reduction launch (partials per slot).
 constexpr int kMaxRedBlocks = 4096;
 
@@ -52,7 +54,7 @@ struct Context
 	bool own_stream = false;
 	int num_sms = 0;
 	// reduction scratch: partials [kSlots][kMaxRedBlocks] (double),
-	// results [kSlots] (double), counters [kSlots] (unsigned)
+	// results [kSlots] (double), counters [kCounters] (unsigned, zero between launches)
 	double *d_partials = nullptr;
 	double *d_results = nullptr;
 	unsigned *d_counters = nullptr;
@@ -63,10 +65,30 @@ struct Context
 	void *d_stage = nullptr;
 	size_t stage_bytes = 0;
 
-	// scratch of the momentum step on plain fields (md_products.cuh), grown on
-	// demand up to that file's cap
-	void *d_md = nullptr;
-	size_t md_bytes = 0;
+	// workspace of calls on plain fields (products of a momentum step, lines of
+	// Wilson loops): on this context's stream, so calls use it one after another;
+	// grown on demand, freed with the context
+	static constexpr size_t kWorkCap = size_t(512) << 20; // kept between calls at most
+	void *d_work = nullptr;
+	size_t work_bytes = 0;
+	// false (and no workspace) when there is no memory
+	bool grow_work(size_t bytes)
+	{
+		if (work_bytes >= bytes)
+			return true;
+		cudaStreamSynchronize(stream);
+		cudaFree(d_work);
+		d_work = nullptr;
+		work_bytes = 0;
+		if (cudaMalloc(&d_work, bytes) != cudaSuccess)
+		{
+			cudaGetLastError();
+			d_work = nullptr;
+			return false;
+		}
+		work_bytes = bytes;
+		return true;
+	}
 
 	void *stage(size_t bytes)
 	{

@@ -129,9 +129,14 @@ struct OpsTable
 	bool (*hmc_md_step)(Field &P, Field const &Uin, Field &Uout, double coef, double tu, bool reunit, RedSlot *kin,
 	                    MdScratch const &scratch, bool row2);
 	void (*hmc_tune_md)(Field &P, Field const &Uin, Field &Uout, MdScratch const &scratch);
-	// Wilson loops (4D): Lout = Lprev U_dir(x + (n-1) dir); sum of the r x t loops
-	void (*line_extend)(Field const &U, int dir, int n, void const *Lprev, void *Lout);
-	void (*wilson_rt)(Field const &U, int r, int t, void const *S, void const *Tt, RedSlot out);
+	// Wilson loops (4D): the temporal lines of 1 .. max_t links, the spatial lines
+	// grown to r links, and the sums of the r x t loops for t = 1 .. max_t
+	// (partials: wilson_partials doubles; counters: zero, one per chunk of t)
+	size_t (*wilson_partials)(Context const &c, int max_t);
+	void (*temporal_lines)(Field const &U, int max_t, void *lines);
+	void (*spatial_lines)(Field const &U, int r, void *S);
+	void (*wilson_t)(Field const &U, int r, int max_t, void const *S, void const *lines, double *partials,
+	                 unsigned *counters, double *result);
 	// one heat-bath (overrelax = false) or overrelaxation sweep, checkerboard order
 	void (*gauge_sweep)(Field &U, double beta, uint64_t seed, uint64_t ctr, bool overrelax);
 	// layout conversion reading / writing a device-accessible host buffer directly

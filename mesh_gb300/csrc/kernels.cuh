@@ -1337,56 +1337,138 @@ template <int ND> __device__ __forceinline__ int64_t eo_offset(Geom const &g, Si
 	return int64_t(st.par ^ (off & 1)) * g.Vh + (lex >> 1);
 }
 
-// Lout(x) = Lprev(x) U_dir(x + (n - 1) dir): the line of n links from x
-// (Lout may be Lprev: every site reads and writes only its own line)
+// temporal lines T_t(x) = T_{t-1}(x) U_3(x + (t - 1) 3), t = 1 .. max_t, component
+// t - 1 of `lines`: one thread a site carries the product, which is read back by
+// nobody while the lines grow
 template <int GRP, class T, int ND>
-__global__ void __launch_bounds__(kBlock)
-    k_line_extend(Geom g, int dir, int n, T const *Lprev, T const *__restrict__ U, T *Lout)
+__global__ void __launch_bounds__(kBlock) k_temporal_lines(Geom g, int max_t, T const *__restrict__ U, T *__restrict__ lines)
 {
 	using Gp = Group<GRP, T>;
 	using E = typename Gp::E;
-	int off = (n - 1) % g.Ld(dir);
+	T const *U3 = U + int64_t(3) * Gp::NR * g.V;
 	MESH_GRID_LOOP(s, g.V)
 	{
 		Site<ND> st = site_from_eo<ND>(g, s);
-		E a, b;
-		Soa<T, Gp::NR>::load(Lprev, g.V, s, a.v);
-		Soa<T, Gp::NR>::load(U + int64_t(dir) * Gp::NR * g.V, g.V, eo_offset<ND>(g, st, dir, off), b.v);
-		E c = Gp::mul(a, b);
-		Soa<T, Gp::NR>::store(Lout, g.V, s, c.v);
+		E a;
+		Soa<T, Gp::NR>::load(U3, g.V, s, a.v);
+		comp<T, Gp::NR>(lines, g.V, 0).store(s, a.v);
+		for (int t = 2; t <= max_t; ++t)
+		{
+			E b;
+			Soa<T, Gp::NR>::load(U3, g.V, eo_offset<ND>(g, st, 3, t - 1), b.v);
+			a = Gp::mul(a, b);
+			comp<T, Gp::NR>(lines, g.V, t - 1).store(s, a.v);
+		}
 	}
 }
 
-// sum over sites and mu < 3 of ReTr(S_mu(x) T(x + r mu) S_mu(x + t 3)^+ T(x)^+),
-// S: the three spatial lines of r links (components 0..2), T: the line of t
-// links in direction 3
+// spatial lines of direction mu = blockIdx.y, grown in place to r links:
+// S_mu(x) <- S_mu(x) U_mu(x + (r - 1) mu); r = 1 copies the links
 template <int GRP, class T, int ND>
-__global__ void __launch_bounds__(kBlock)
-    k_wilson_rt(Geom g, int r, int t, T const *__restrict__ S, T const *__restrict__ Tt, RedSlot out)
+__global__ void __launch_bounds__(kBlock) k_spatial_lines(Geom g, int r, T const *__restrict__ U, T *__restrict__ S)
 {
 	using Gp = Group<GRP, T>;
 	using E = typename Gp::E;
-	double acc = 0.0;
+	int mu = blockIdx.y;
+	auto Sv = comp<T, Gp::NR>(S, g.V, mu);
 	MESH_GRID_LOOP(s, g.V)
 	{
-		Site<ND> st = site_from_eo<ND>(g, s);
-		E d;
-		Soa<T, Gp::NR>::load(Tt, g.V, s, d.v);
-		int64_t xt = eo_offset<ND>(g, st, 3, t % g.Ld(3));
-		T sum = T(0);
-#pragma unroll 1
-		for (int mu = 0; mu < 3; ++mu)
+		E a, b;
+		if (r == 1)
+			comp<T, Gp::NR>(const_cast<T *>(U), g.V, mu).load(s, a.v);
+		else
 		{
-			T const *Smu = S + int64_t(mu) * Gp::NR * g.V;
-			E a, b, c;
-			Soa<T, Gp::NR>::load(Smu, g.V, s, a.v);
-			Soa<T, Gp::NR>::load(Tt, g.V, eo_offset<ND>(g, st, mu, r % g.Ld(mu)), b.v);
-			Soa<T, Gp::NR>::load(Smu, g.V, xt, c.v);
-			sum += Gp::retr_nd(Gp::mul(a, b), Gp::mul(d, c));
+			Site<ND> st = site_from_eo<ND>(g, s);
+			Sv.load(s, a.v);
+			comp<T, Gp::NR>(const_cast<T *>(U), g.V, mu).load(eo_offset<ND>(g, st, mu, (r - 1) % g.Ld(mu)), b.v);
+			a = Gp::mul(a, b);
 		}
-		acc += double(sum);
+		Sv.store(s, a.v);
 	}
-	grid_sum<kBlock>(acc, out);
+}
+
+// W(r, t) for the chunk of kWilsonT extents t that blockIdx.y names: the sums over
+// sites and mu < 3 of ReTr(S_mu(x) T_t(x + r mu) S_mu(x + t 3)^+ T_t(x)^+), S: the
+// spatial lines of r links, Tl: the temporal lines. Tiles of 32 sites, one warp per
+// mu: S_mu(x) stays in registers for the chunk, S_mu(x + t 3) comes from the same
+// x3 lines for every t and T_t(x) serves the three warps, both mostly from L1. What
+// bounds it is L2 to L1 (about 9 TB/s): a launch for each (r, t) read ten links a
+// site from L2, here it is a good half.
+// 24^4 SU(3) FP32 on a GB300, t = 1 .. 12 of one r: 379 us in a launch each, 240
+// here. Measured and not kept: chunks of 8 and 12 (264, 305 us), six or more blocks
+// per SM under fewer registers (289 to 353), blocks that walk whole planes (mu, 3)
+// with t inside (283 to 348) or outside (352 to 600) the loop over sites.
+constexpr int kWilsonT = 4;
+template <int GRP, class T, int ND>
+__global__ void __launch_bounds__(96, sizeof(T) == 8 ? 3 : 5)
+    k_wilson_t(Geom g, int r, int max_t, T const *__restrict__ S, T const *__restrict__ Tl, double *__restrict__ partials,
+               unsigned *counters, double *__restrict__ result)
+{
+	using Gp = Group<GRP, T>;
+	using E = typename Gp::E;
+	__shared__ double sw[3][kWilsonT];
+	__shared__ bool is_last;
+	int mu = threadIdx.x >> 5, lane = threadIdx.x & 31;
+	int t0 = 1 + int(blockIdx.y) * kWilsonT, nt = max_t + 1 - t0 < kWilsonT ? max_t + 1 - t0 : kWilsonT;
+	auto Sv = comp<T, Gp::NR>(const_cast<T *>(S), g.V, mu);
+	double acc[kWilsonT];
+#pragma unroll
+	for (int k = 0; k < kWilsonT; ++k)
+		acc[k] = 0.0;
+	int ntiles = slab_tiles(g.V, 1);
+	for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x)
+	{
+		int64_t s;
+		if (!slab_site(g, g.V, 0, 1, tile, s))
+			continue;
+		Site<ND> st = site_from_eo<ND>(g, s);
+		E a;
+		Sv.load(s, a.v);
+		int64_t xr = eo_offset<ND>(g, st, mu, r % g.Ld(mu));
+#pragma unroll
+		for (int k = 0; k < kWilsonT; ++k)
+			if (k < nt)
+			{
+				int t = t0 + k;
+				auto Tv = comp<T, Gp::NR>(const_cast<T *>(Tl), g.V, t - 1);
+				E b, c, d;
+				Tv.load(xr, b.v);
+				Tv.load(s, d.v);
+				Sv.load(eo_offset<ND>(g, st, 3, t % g.Ld(3)), c.v);
+				acc[k] += double(Gp::retr_nd(Gp::mul(a, b), Gp::mul(d, c)));
+			}
+	}
+#pragma unroll
+	for (int k = 0; k < kWilsonT; ++k)
+	{
+		double v = warp_sum(acc[k]);
+		if (lane == 0)
+			sw[mu][k] = v;
+	}
+	__syncthreads();
+	// the block's sums; the last block of the chunk adds them in a fixed order
+	double *part = partials + int64_t(blockIdx.y) * kWilsonT * gridDim.x;
+	if (threadIdx.x < kWilsonT)
+	{
+		part[int64_t(threadIdx.x) * gridDim.x + blockIdx.x] = (sw[0][threadIdx.x] + sw[1][threadIdx.x]) + sw[2][threadIdx.x];
+		__threadfence();
+	}
+	__syncthreads();
+	if (threadIdx.x == 0)
+		is_last = atomicInc(counters + blockIdx.y, gridDim.x - 1) == gridDim.x - 1;
+	__syncthreads();
+	if (!is_last)
+		return;
+	__threadfence();
+	for (int k = mu; k < nt; k += 3)
+	{
+		double v = 0.0;
+		for (unsigned b = lane; b < gridDim.x; b += 32)
+			v += __ldcg(part + int64_t(k) * gridDim.x + b);
+		v = warp_sum(v);
+		if (lane == 0)
+			result[t0 - 1 + k] = v;
+	}
 }
 
 template <int GRP, class T, int ND>
@@ -2898,24 +2980,43 @@ template <int GRP, class T, int ND> struct Ops
 				MESH_LAUNCH_CHECK();
 			}
 	}
-	// Wilson loops: one line extension / the r x t loop sum (4D only)
-	static void line_extend(Field const &U, int dir, int n, void const *Lprev, void *Lout)
+	// Wilson loops (4D only): the temporal lines, the spatial lines of r links, the
+	// sums of all extents t (partials: wilson_partials doubles)
+	static constexpr int kWilsonBlocks = 5; // blocks per SM of a chunk of extents
+	static size_t wilson_partials(Context const &c, int max_t)
+	{
+		return size_t((max_t + kWilsonT - 1) / kWilsonT) * kWilsonT * size_t(c.num_sms) * kWilsonBlocks;
+	}
+	static void temporal_lines(Field const &U, int max_t, void *lines)
 	{
 		if constexpr (ND == 4)
 		{
 			auto &c = *U.ctx;
-			k_line_extend<GRP, T, ND><<<blocks(c, U.geom.V), kBlock, 0, c.stream>>>(
-			    U.geom, dir, n, static_cast<T const *>(Lprev), static_cast<T const *>(U.d), static_cast<T *>(Lout));
+			k_temporal_lines<GRP, T, ND><<<blocks(c, U.geom.V), kBlock, 0, c.stream>>>(
+			    U.geom, max_t, static_cast<T const *>(U.d), static_cast<T *>(lines));
 			MESH_LAUNCH_CHECK();
 		}
 	}
-	static void wilson_rt(Field const &U, int r, int t, void const *S, void const *Tt, RedSlot out)
+	static void spatial_lines(Field const &U, int r, void *S)
 	{
 		if constexpr (ND == 4)
 		{
 			auto &c = *U.ctx;
-			k_wilson_rt<GRP, T, ND><<<red_blocks(c, U.geom.V), kBlock, 0, c.stream>>>(
-			    U.geom, r, t, static_cast<T const *>(S), static_cast<T const *>(Tt), out);
+			k_spatial_lines<GRP, T, ND><<<dim3(blocks(c, U.geom.V), 3), kBlock, 0, c.stream>>>(
+			    U.geom, r, static_cast<T const *>(U.d), static_cast<T *>(S));
+			MESH_LAUNCH_CHECK();
+		}
+	}
+	static void wilson_t(Field const &U, int r, int max_t, void const *S, void const *lines, double *partials,
+	                     unsigned *counters, double *result)
+	{
+		if constexpr (ND == 4)
+		{
+			auto &c = *U.ctx;
+			int64_t tiles = slab_tiles(U.geom.V, 1), cap = int64_t(c.num_sms) * kWilsonBlocks;
+			dim3 grid(unsigned(tiles < cap ? tiles : cap), unsigned((max_t + kWilsonT - 1) / kWilsonT));
+			k_wilson_t<GRP, T, ND><<<grid, 96, 0, c.stream>>>(U.geom, r, max_t, static_cast<T const *>(S),
+			                                                  static_cast<T const *>(lines), partials, counters, result);
 			MESH_LAUNCH_CHECK();
 		}
 	}
@@ -2927,7 +3028,7 @@ template <int GRP, class T, int ND> struct Ops
 		                           landau_theta, landau_deriv,  landau_or_half, reunit_exact,   alg_dot,
 		                           exp_apply,    axpy_alg,      gauge_transform,
 		                           hmc_plaquette, hmc_evolve,   hmc_momentum_step,
-		                           hmc_md_step,   hmc_tune_md,  line_extend,    wilson_rt,
+		                           hmc_md_step,   hmc_tune_md,  wilson_partials, temporal_lines, spatial_lines, wilson_t,
 		                           gauge_sweep,   import_direct, export_direct, md_scratch_bytes};
 		return &t;
 	}

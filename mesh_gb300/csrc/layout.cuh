@@ -156,6 +156,18 @@ template <int ND> __device__ __forceinline__ int64_t eo_of(Geom const &g, Site<N
 	return int64_t(st.par) * g.Vh + (st.lex >> 1);
 }
 
+// tiles of 32 sites of n slices of dimension 0, S sites each; tile 2j holds the j-th 32 even sites, 2j + 1 the
+// odd ones beside them (all even sites first read every neighbour link, of odd
+// sites, long before the odd sites did: twice the DRAM traffic)
+__host__ __device__ __forceinline__ int slab_tiles(int64_t S, int n) { return 2 * int((n * (S / 2) + 31) / 32); }
+// this lane's site of a tile of the slices [x0, x0 + n), false past the end
+__device__ __forceinline__ bool slab_site(Geom const &g, int64_t S, int x0, int n, int tile, int64_t &s)
+{
+	int32_t j = (tile >> 1) * 32 + int32_t(threadIdx.x & 31), h = int32_t(S / 2);
+	s = int64_t(tile & 1) * g.Vh + int64_t(x0) * h + j;
+	return j < n * h;
+}
+
 // lexicographic index after a step of `sign` (+-1) in direction dir
 __device__ __forceinline__ int32_t lex_step(Geom const &g, uint32_t px, int32_t lex, int dir, int sign)
 {

@@ -48,18 +48,6 @@ __device__ __forceinline__ int64_t ring_index(MdRing const &r, int32_t lex, int 
 	return int64_t(par) * (r.V / 2) + (l >> 1);
 }
 
-// tiles of 32 sites of n slices; tile 2j holds the j-th 32 even sites, 2j + 1 the
-// odd ones beside them (all even sites first read every neighbour link, of odd
-// sites, long before the odd sites did: twice the DRAM traffic)
-__host__ __device__ __forceinline__ int slab_tiles(int64_t S, int n) { return 2 * int((n * (S / 2) + 31) / 32); }
-// this lane's site of a tile of the slices [x0, x0 + n), false past the end
-__device__ __forceinline__ bool slab_site(Geom const &g, int64_t S, int x0, int n, int tile, int64_t &s)
-{
-	int32_t j = (tile >> 1) * 32 + int32_t(threadIdx.x & 31), h = int32_t(S / 2);
-	s = int64_t(tile & 1) * g.Vh + int64_t(x0) * h + j;
-	return j < n * h;
-}
-
 // products of the slices [x0, x0 + n) into the ring, slice x0 at t = t0
 template <class T, int ND>
 __global__ void __launch_bounds__(32 * kPlanes<ND>)

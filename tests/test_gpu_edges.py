@@ -140,3 +140,14 @@ def test_fp32_su3_step_from_plaquettes_in_slabs(ctx):
     assert "stored plaquettes" in [ln for ln in mg.tune_report().splitlines() if "md_step/group3/f32/40x32x34x32" in ln][0]
     assert rel(ua, ub) < 2e-5 and rel(pa, pb) < 2e-5
     assert ra["H_new"] == pytest.approx(rb["H_new"], rel=1e-6)
+
+
+@pytest.mark.parametrize("max_t", [1, 3, 4, 5, 14])
+@pytest.mark.parametrize("g,p", [(1, 1), (2, 2), (3, 2), (3, 1)])
+def test_wilson_loops_in_chunks(ctx, oracle, g, p, max_t):
+    """extents t on both sides of a chunk, tiles with missing sites"""
+    dims = [2, 6, 4, 14]
+    U64 = links(oracle, g, dims)
+    U = mg.GaugeField(ctx, g, p, mg.Grid(dims)).import_(U64.astype(mg.real_dtype(p)))
+    W = mg.wilson_loops(U, 2, max_t)
+    assert np.max(np.abs(W - oracle.wilson_loops(g, 2, dims, U64, 2, max_t))) < (1e-13 if p == 2 else 2e-6)
