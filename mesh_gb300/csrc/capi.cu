@@ -332,7 +332,7 @@ struct mesh_hmc_s
 	int *d_flag = nullptr;
 	int64_t count = 0; // trajectories enqueued
 	bool S_valid = false;
-	// products of a momentum step (allocated by the first step outside a capture)
+	// products or plaquettes of a momentum step
 	MdScratch scratch;
 	// cached CUDA graph of one trajectory
 	cudaGraphExec_t graph = nullptr;
@@ -379,12 +379,11 @@ struct mesh_hmc_s
 		drop_graph();
 	}
 
-	// the chain's scratch, before its first step; a chain without the memory
-	// for it steps without it
-	void ensure_scratch()
+	// the chain's scratch; a chain without the memory for it steps without it
+	void make_scratch()
 	{
 		size_t need = ops_for(U.f).md_scratch_bytes(U.f.geom, true);
-		if (need == 0 || scratch.d || capturing(*ctx))
+		if (need == 0)
 			return;
 		if (cudaMalloc(&scratch.d, need) == cudaSuccess)
 			scratch.bytes = need;
@@ -402,7 +401,6 @@ struct mesh_hmc_s
 		Field &u = U.f, &un = Unew.f, &p = P.f;
 		auto const &ops = ops_for(u);
 		Context &c = *ctx;
-		ensure_scratch();
 		if (!S_valid)
 		{
 			ops.hmc_plaquette(u, rs(S_CUR));
@@ -1013,12 +1011,43 @@ int mesh_run_hmd(mesh_field Uh, mesh_field Ph, double beta, double const *deltas
 		DeviceGuard dg(U.ctx->device);
 		auto const &ops = ops_for(U);
 		double coef0 = beta / (2.0 * group_nc(U.group));
-		MdScratch scratch = ctx_md_scratch(U);
-		for (int i = 0; i < n; ++i)
-			if (i % 2 == 0)
-				ops.evolve(U, U, P, deltas[i], false);
-			else
-				ops.momentum_step(P, U, coef0 * deltas[i], nullptr, scratch);
+		// Momentum steps fused with the link updates after them write the links out
+		// of place: a second buffer from the workspace beside the step's scratch. The
+		// fused kernels of FP32 SU(3) take special unitary links, which a plain field
+		// need not hold.
+		Context &c = *U.ctx;
+		size_t need = ops.md_scratch_bytes(U.geom, false), at = (need + 255) / 256 * 256;
+		bool fuse = (U.group != 3 || U.prec == MESH_F64) && n >= 3 && !capturing(c) &&
+		            at + U.bytes <= Context::kWorkCap && c.grow_work(at + U.bytes);
+		if (!fuse)
+		{
+			MdScratch scratch = ctx_md_scratch(U);
+			for (int i = 0; i < n; ++i)
+				if (i % 2 == 0)
+					ops.evolve(U, U, P, deltas[i], false);
+				else
+					ops.momentum_step(P, U, coef0 * deltas[i], nullptr, scratch);
+			return;
+		}
+		MdScratch scratch{c.d_work, at};
+		Field W = U; // U's shape on the workspace
+		W.d = static_cast<char *>(c.d_work) + at;
+		// an even number of changes of buffer ends in U
+		int steps = n / 2;
+		Field *cur = &U, *spare = &W;
+		Field first = U;
+		if (steps % 2)
+			std::swap(cur, spare);
+		ops.evolve(first, *cur, P, deltas[0], false);
+		for (int i = 1; i < n; i += 2)
+		{
+			if (!ops.hmc_md_step(P, *cur, *spare, coef0 * deltas[i], deltas[i + 1], false, nullptr, scratch, true))
+			{
+				ops.momentum_step(P, *cur, coef0 * deltas[i], nullptr, scratch);
+				ops.evolve(*cur, *spare, P, deltas[i + 1], false);
+			}
+			std::swap(cur, spare);
+		}
 	});
 }
 
@@ -1062,6 +1091,7 @@ int mesh_hmc_create(mesh_ctx ctx, int group, int precision, int nd, int32_t cons
 		MESH_CUDA(cudaMemset(h->d_cnt, 0, sizeof(unsigned) * mesh_hmc_s::NSLOT));
 		MESH_CUDA(cudaMemset(h->d_res, 0, sizeof(double) * mesh_hmc_s::NSLOT));
 		h->ensure_history(1024);
+		h->make_scratch();
 		ops_for(h->U.f).set_unit(h->U.f);
 	});
 	if (rc != MESH_OK)
@@ -1176,7 +1206,6 @@ int mesh_hmc_momentum_step(mesh_hmc h, double beta, double delta)
 		require(h != nullptr, "null hmc");
 		DeviceGuard dg(h->ctx->device);
 		Field &U = h->U.f, &P = h->P.f;
-		h->ensure_scratch();
 		ops_for(U).hmc_momentum_step(P, U, beta / (2.0 * group_nc(U.group)) * delta, nullptr, h->scratch);
 	});
 }
@@ -1188,7 +1217,6 @@ int mesh_hmc_md_step(mesh_hmc h, double beta, double dp, double du)
 		DeviceGuard dg(h->ctx->device);
 		Field &U = h->U.f, &P = h->P.f;
 		auto const &ops = ops_for(U);
-		h->ensure_scratch();
 		double coef = beta / (2.0 * group_nc(U.group)) * dp;
 		if (ops.hmc_md_step(P, U, h->Ut.f, coef, du, false, nullptr, h->scratch, true))
 		{
@@ -1271,7 +1299,6 @@ int mesh_hmc_run(mesh_hmc h, double beta, double const *deltas, int n, int count
 			ops_for(h->U.f).hmc_plaquette(h->U.f, h->rs(mesh_hmc_s::S_CUR));
 			h->S_valid = true;
 		}
-		h->ensure_scratch();
 		// choose launch variants before capturing (tuning times kernels)
 		ops_for(h->U.f).hmc_tune_md(h->P.f, h->Unew.f, h->Ut.f, h->scratch);
 		std::vector<double> dv(deltas, deltas + n);

@@ -790,48 +790,47 @@ template <int ND, int NA, class T> __device__ __forceinline__ void add_dir(T (&F
 		}
 }
 
-// The per-site body for the small groups (U(1), SU(2)) in four dimensions:
-// the same momentum step (and with FUSE link update) as site_md below,
-// unrolled over planes and directions, with the site's four own links held in
-// registers and the twenty neighbour indices (x + e_mu, x - e_nu,
-// x - e_nu + e_mu) computed once per site instead of once per staple: for
-// these groups the products are a few FMAs, and the index arithmetic, not the
-// arithmetic of the staples, set the instruction count.
-template <int GRP, class T, bool FUSE, class LD>
-__device__ __forceinline__ double site_md_small(Geom const &g, Site<4> const &st, int64_t s, LD const &ld,
+// The per-site body for the small groups (U(1), SU(2)): the same momentum step (and
+// with FUSE link update) as site_md below, unrolled over planes and directions,
+// with the site's own links held in registers and the neighbour indices (twenty in
+// four dimensions: x + e_mu, x - e_nu, x - e_nu + e_mu) computed once per site
+// instead of once per staple: for these groups the products are a few FMAs, and the
+// index arithmetic, not the arithmetic of the staples, set the instruction count.
+template <int GRP, class T, int ND, bool FUSE, class LD>
+__device__ __forceinline__ double site_md_small(Geom const &g, Site<ND> const &st, int64_t s, LD const &ld,
                                                 T *__restrict__ P, T coef, T *__restrict__ Uout, T tu, int reunit,
                                                 bool want_kin)
 {
 	using Gp = Group<GRP, T>;
 	using E = typename Gp::E;
 	constexpr int NA = Gp::NA;
-	int32_t f[4], b[4], d[4][4];
+	int32_t f[ND], b[ND], d[ND][ND];
 #pragma unroll
-	for (int mu = 0; mu < 4; ++mu)
+	for (int mu = 0; mu < ND; ++mu)
 	{
-		f[mu] = int32_t(eo_shift1<4>(g, st, mu, +1));
-		b[mu] = int32_t(eo_shift1<4>(g, st, mu, -1));
+		f[mu] = int32_t(eo_shift1<ND>(g, st, mu, +1));
+		b[mu] = int32_t(eo_shift1<ND>(g, st, mu, -1));
 	}
 #pragma unroll
-	for (int nu = 0; nu < 4; ++nu)
+	for (int nu = 0; nu < ND; ++nu)
 #pragma unroll
-		for (int mu = 0; mu < 4; ++mu)
-			d[nu][mu] = mu == nu ? 0 : int32_t(eo_shift2<4>(g, st, nu, -1, mu, +1));
-	E u[4];
+		for (int mu = 0; mu < ND; ++mu)
+			d[nu][mu] = mu == nu ? 0 : int32_t(eo_shift2<ND>(g, st, nu, -1, mu, +1));
+	E u[ND];
 #pragma unroll
-	for (int mu = 0; mu < 4; ++mu)
+	for (int mu = 0; mu < ND; ++mu)
 		u[mu] = ld(mu, s);
-	T F[4][NA];
+	T F[ND][NA];
 #pragma unroll
-	for (int mu = 0; mu < 4; ++mu)
+	for (int mu = 0; mu < ND; ++mu)
 #pragma unroll
 		for (int a = 0; a < NA; ++a)
 			F[mu][a] = T(0);
 	// forward plaquette loops: (a b)(d c)^+ closes both forward staples
 #pragma unroll
-	for (int mu = 0; mu < 4; ++mu)
+	for (int mu = 0; mu < ND; ++mu)
 #pragma unroll
-		for (int nu = mu + 1; nu < 4; ++nu)
+		for (int nu = mu + 1; nu < ND; ++nu)
 		{
 			E pl = Gp::mul_nd(Gp::mul(u[mu], ld(nu, f[mu])), Gp::mul(u[nu], ld(mu, f[nu])));
 			T xa[NA];
@@ -845,11 +844,11 @@ __device__ __forceinline__ double site_md_small(Geom const &g, Site<4> const &st
 		}
 	// lower staples, summed per link and closed with U_mu(x)
 #pragma unroll
-	for (int mu = 0; mu < 4; ++mu)
+	for (int mu = 0; mu < ND; ++mu)
 	{
 		E S = Gp::zero();
 #pragma unroll
-		for (int nu = 0; nu < 4; ++nu)
+		for (int nu = 0; nu < ND; ++nu)
 		{
 			if (nu == mu)
 				continue;
@@ -863,7 +862,7 @@ __device__ __forceinline__ double site_md_small(Geom const &g, Site<4> const &st
 	}
 	T kacc = T(0); // the site's kinetic terms in the field precision, one FP64 add per site
 #pragma unroll
-	for (int mu = 0; mu < 4; ++mu)
+	for (int mu = 0; mu < ND; ++mu)
 	{
 		auto Pv = comp<T, NA>(P, g.V, mu);
 		T p[NA];
@@ -979,7 +978,7 @@ __device__ __forceinline__ double site_md(Geom const &g, Site<ND> const &st, int
 {
 	// GENERIC: the rolled plane/staple loops below for every group
 	if constexpr (GRP != SU3 && ND == 4 && !SM && !PIPE && !GENERIC)
-		return site_md_small<GRP, T, FUSE>(g, st, s, ld, P, coef, Uout, tu, reunit, want_kin);
+		return site_md_small<GRP, T, ND, FUSE>(g, st, s, ld, P, coef, Uout, tu, reunit, want_kin);
 	using Gp = Group<GRP, T>;
 	using E = typename Gp::E;
 	using Pr = Prod<GRP, T, F2>;
@@ -1229,6 +1228,33 @@ __global__ void __launch_bounds__(NT, MINB)
 	}
 	if (kin.result)
 		grid_sum<NT>(acc, kin);
+}
+
+// The thread-per-site step of U(1) and SU(2) for any extents and dimensions: tiles
+// of 32 sites, even and odd ones in turn. A thread per link recomputes the index
+// arithmetic of every staple, which is most of its instructions for these groups.
+// U(1) FP32 64x96x80 on a GB300: momentum step 25.9 us a thread per link;
+// fused with the link update (7.6 us on its own) 16 us here.
+template <int GRP, class T, int ND, bool FUSE>
+__global__ void __launch_bounds__(128)
+    k_md_small(Geom g, T const *__restrict__ U, T *__restrict__ P, T coef, RedSlot kin, T *__restrict__ Uout, T tu,
+               int reunit)
+{
+	LinkLoad<GRP, T, ND> ld{U, g.V};
+	double acc = 0.0;
+	int ntiles = slab_tiles(g.V, 1);
+	for (int tile = int(blockIdx.x) * 4 + int(threadIdx.x >> 5); tile < ntiles; tile += int(gridDim.x) * 4)
+	{
+		int64_t s;
+		if (!slab_site(g, g.V, 0, 1, tile, s))
+			continue;
+		Site<ND> st = site_from_eo<ND>(g, s);
+		double k = site_md_small<GRP, T, ND, FUSE>(g, st, s, ld, P, coef, Uout, tu, reunit, kin.result != nullptr);
+		if (kin.result)
+			acc += k;
+	}
+	if (kin.result)
+		grid_sum<128>(acc, kin);
 }
 
 // ---------------------------------------------------------------------------
@@ -2165,9 +2191,10 @@ template <int GRP, class T, int ND> struct Ops
 	// selects (1 forward loops, 2 lower staples, 4 link update); 46-48:
 	// thread per site with the next step's neighbour rows copied to shared
 	// memory by cp.async; 49-53, 54-57: thread per site, more tile shapes of
-	// 512 and 256 sites
-	static constexpr int kForceVariants = 58;
-	static int n_force_variants() { return ND == 4 ? kForceVariants : 2; }
+	// 512 and 256 sites; 58: thread per site of U(1) and SU(2), any lattice
+	// (k_md_small)
+	static constexpr int kForceVariants = 59;
+	static int n_force_variants() { return kForceVariants; }
 	static ForceVariant force_variant(int v)
 	{
 		static const ForceVariant t[kForceVariants] = {
@@ -2228,7 +2255,8 @@ template <int GRP, class T, int ND> struct Ops
 		    {2, {0, 1, 4, 4}, 512, 1, "site/tile1x2x16x16/512thr/1blk/f32x2", 1},
 		    {2, {1, 1, 2, 5}, 512, 1, "site/tile2x2x4x32/512thr/1blk/f32x2", 1},
 		    {2, {0, 2, 2, 5}, 512, 1, "site/tile1x4x4x32/512thr/1blk/f32x2", 1},
-		    {2, {0, 1, 3, 5}, 512, 1, "site/tile1x2x8x32/512thr/1blk/f32x2", 1}};
+		    {2, {0, 1, 3, 5}, 512, 1, "site/tile1x2x8x32/512thr/1blk/f32x2", 1},
+		    {4, {0, 0, 0, 0}, 128, 1, "site/eo-order/128thr"}};
 		return t[v];
 	}
 	static bool force_variant_valid(Geom const &g, int v)
@@ -2240,6 +2268,8 @@ template <int GRP, class T, int ND> struct Ops
 			return false;
 		if (!fv.tiled)
 			return true;
+		if (fv.tiled == 4)
+			return GRP != SU3;
 		if (fv.tiled == 3)
 			return GRP == SU3 && ND == 4 && line_supported(g) && (!fv.st || (kF2 && g.L[3] == 32));
 		if (ND != 4)
@@ -2265,6 +2295,11 @@ template <int GRP, class T, int ND> struct Ops
 		ForceVariant fv = force_variant(v);
 		T const *u = static_cast<T const *>(U.d);
 		T *p = static_cast<T *>(P.d);
+		if (fv.tiled == 4)
+		{
+			launch_small<false>(g, u, p, coef, kin, c, nullptr, T(0), 0);
+			return;
+		}
 		if (!fv.tiled)
 		{
 			int64_t n = int64_t(ND) * g.V;
@@ -2313,6 +2348,18 @@ template <int GRP, class T, int ND> struct Ops
 				k_momentum_step_tiled<GRP, T, 4, 128, 4, false, ROWS><<<b, 128, 0, c.stream>>>(g, ts, u, p, coef, kin);
 		}
 		MESH_LAUNCH_CHECK();
+	}
+	template <bool FUSE>
+	static void launch_small(Geom const &g, T const *u, T *p, T coef, RedSlot kin, Context &c, T *uo, T tu, int reunit)
+	{
+		if constexpr (GRP != SU3)
+		{
+			auto k = k_md_small<GRP, T, ND, FUSE>;
+			unsigned b = resident_grid(c, k, 128, (slab_tiles(g.V, 1) + 3) / 4);
+			k<<<b < unsigned(kMaxRedBlocks) ? b : unsigned(kMaxRedBlocks), 128, 0, c.stream>>>(g, u, p, coef, kin, uo, tu,
+			                                                                                 reunit);
+			MESH_LAUNCH_CHECK();
+		}
 	}
 	template <bool ROWS>
 	static void launch_force_site(ForceVariant const &fv, unsigned b, Geom const &g, TileSpec const &ts, T const *u,
@@ -2618,11 +2665,9 @@ template <int GRP, class T, int ND> struct Ops
 		}
 	}
 	// ---- fused momentum step + link update (trajectory) ----------------------
-	static constexpr int kMdFirst = 14, kMdLast = 57; // thread-per-site and line-march variants
+	static constexpr int kMdFirst = 14, kMdLast = 58; // thread-per-site and line-march variants
 	static bool md_supported(Geom const &g)
 	{
-		if constexpr (ND != 4)
-			return false;
 		for (int v = kMdFirst; v <= kMdLast; ++v)
 			if (force_variant_valid(g, v))
 				return true;
@@ -2635,7 +2680,10 @@ template <int GRP, class T, int ND> struct Ops
 	template <bool R>
 	static void launch_md_t(int v, Field &P, Field const &Uin, Field &Uout, T coef, T tu, int reunit, RedSlot kin)
 	{
-		if constexpr (ND == 4)
+		if (force_variant(v).tiled == 4)
+			launch_small<true>(Uin.geom, static_cast<T const *>(Uin.d), static_cast<T *>(P.d), coef, kin, *Uin.ctx,
+			                   static_cast<T *>(Uout.d), tu, reunit);
+		else if constexpr (ND == 4)
 		{
 			auto &c = *Uin.ctx;
 			Geom const &g = Uin.geom;

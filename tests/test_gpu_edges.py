@@ -151,3 +151,20 @@ def test_wilson_loops_in_chunks(ctx, oracle, g, p, max_t):
     U = mg.GaugeField(ctx, g, p, mg.Grid(dims)).import_(U64.astype(mg.real_dtype(p)))
     W = mg.wilson_loops(U, 2, max_t)
     assert np.max(np.abs(W - oracle.wilson_loops(g, 2, dims, U64, 2, max_t))) < (1e-13 if p == 2 else 2e-6)
+
+
+@pytest.mark.parametrize("steps", [1, 2])
+@pytest.mark.parametrize("dims", SHAPES, ids=lambda d: "x".join(map(str, d)))
+@pytest.mark.parametrize("g,p", [(1, 1), (1, 2), (2, 1), (2, 2), (3, 1), (3, 2)])
+def test_run_hmd_fused_steps(ctx, oracle, g, p, dims, steps):
+    """momentum steps fused with link updates out of place (an odd and an even
+    number of buffer changes) end in U and P"""
+    U64, P64 = links(oracle, g, dims), oracle.random_momenta(g, 2, dims, 11, 0)
+    dt = mg.real_dtype(p)
+    U = mg.GaugeField(ctx, g, p, mg.Grid(dims)).import_(U64.astype(dt))
+    P = mg.Momenta(ctx, g, p, mg.Grid(dims)).import_(P64.astype(dt))
+    d = oracle.make_deltas("2lf", 0.02, steps)
+    mg.run_hmd(U, P, 2.0 * g, d)
+    Uo, Po = oracle.run_hmd(g, 2, dims, U64, P64, 2.0 * g, d)
+    tol = 1e-12 if p == 2 else 2e-5
+    assert rel(U.export(), Uo) < tol and rel(P.export(), Po) < tol
