@@ -64,8 +64,17 @@ template <class T> MESH_HD void m_sincos(T x, T *s, T *c)
 #ifdef __CUDA_ARCH__
 template <> __device__ __forceinline__ void m_sincos<float>(float x, float *s, float *c) { sincosf(x, s, c); }
 template <> __device__ __forceinline__ void m_sincos<double>(double x, double *s, double *c) { sincos(x, s, c); }
-template <> __device__ __forceinline__ double m_rsqrt<double>(double x) { return rsqrt(x); }
 #endif
+// 1 / sqrt(x), in FP64 on the device in half the operations of the square root and
+// the division
+template <class T> MESH_HD T m_rsqrt_fast(T x)
+{
+#ifdef __CUDA_ARCH__
+	if constexpr (sizeof(T) == 8)
+		return rsqrt(x);
+#endif
+	return m_rsqrt(x);
+}
 
 enum
 {
@@ -293,7 +302,10 @@ template <class T> struct Group<SU3, T>
 	// FP64 operation at a small fraction of the FP32 rate, so every FP64 kernel
 	// of SU(3) is bound by their number. FP32 products keep the pairs: their
 	// hot users have packed forms (Su3F2), and the heat-bath's accept tests
-	// compare draws with what these roundings give.
+	// compare draws with what these roundings give. So do the FP64 links and
+	// updates of Fourier-accelerated gauge fixing (mul_pairs, mul_nd_pairs,
+	// exp_alg_closed): its step goes through an FP32 transform, where one Delta
+	// that rounds to another float moves the result by 1e-8 after a few steps.
 	static constexpr bool kChain = sizeof(T) == 8;
 	// r (ADD: += ) sum_k A(i, k) B(k, j) for the rows i < NRW
 	template <int NRW, bool ADD, class FA, class FB> MESH_HD static void chain(E &r, FA A, FB B)
@@ -334,15 +346,10 @@ template <class T> struct Group<SU3, T>
 	{
 		chain<3, true>(s, [&](int i, int k) { return cconj(b.at(k, i)); }, [&](int k, int j) { return cconj(a.at(j, k)); });
 	}
-	// c = a * b
-	MESH_HD static E mul(E const &a, E const &b)
+	// c = a * b from pairs of terms (see kChain)
+	MESH_HD static E mul_pairs(E const &a, E const &b)
 	{
 		E r;
-		if constexpr (kChain)
-		{
-			chain<3, false>(r, [&](int i, int k) { return a.at(i, k); }, [&](int k, int j) { return b.at(k, j); });
-			return r;
-		}
 #pragma unroll
 		for (int i = 0; i < 3; ++i)
 #pragma unroll
@@ -361,6 +368,18 @@ template <class T> struct Group<SU3, T>
 			}
 		return r;
 	}
+	// c = a * b
+	MESH_HD static E mul(E const &a, E const &b)
+	{
+		if constexpr (kChain)
+		{
+			E r;
+			chain<3, false>(r, [&](int i, int k) { return a.at(i, k); }, [&](int k, int j) { return b.at(k, j); });
+			return r;
+		}
+		else
+			return mul_pairs(a, b);
+	}
 	// c = a * b for special unitary a, b: rows 0 and 1 of the product (only
 	// rows 0 and 1 of a are read), row 2 rebuilt as conj(row 0 x row 1)
 	MESH_HD static E mul_r2(E const &a, E const &b)
@@ -372,33 +391,31 @@ template <class T> struct Group<SU3, T>
 			complete_row2(r);
 			return r;
 		}
-#pragma unroll
-		for (int i = 0; i < 2; ++i)
-#pragma unroll
-			for (int j = 0; j < 3; ++j)
-			{
-				T re = 0, im = 0;
-#pragma unroll
-				for (int k = 0; k < 3; ++k)
-				{
-					re += a.v[6 * i + 2 * k] * b.v[6 * k + 2 * j] - a.v[6 * i + 2 * k + 1] * b.v[6 * k + 2 * j + 1];
-					im += a.v[6 * i + 2 * k] * b.v[6 * k + 2 * j + 1] + a.v[6 * i + 2 * k + 1] * b.v[6 * k + 2 * j];
-				}
-				r.v[6 * i + 2 * j] = re;
-				r.v[6 * i + 2 * j + 1] = im;
-			}
-		complete_row2(r);
-		return r;
-	}
-	// c = a * b^dagger:  c_ij = sum_k a_ik conj(b_jk)
-	MESH_HD static E mul_nd(E const &a, E const &b)
-	{
-		E r;
-		if constexpr (kChain)
+		else
 		{
-			chain<3, false>(r, [&](int i, int k) { return a.at(i, k); }, [&](int k, int j) { return cconj(b.at(j, k)); });
+#pragma unroll
+			for (int i = 0; i < 2; ++i)
+#pragma unroll
+				for (int j = 0; j < 3; ++j)
+				{
+					T re = 0, im = 0;
+#pragma unroll
+					for (int k = 0; k < 3; ++k)
+					{
+						re += a.v[6 * i + 2 * k] * b.v[6 * k + 2 * j] - a.v[6 * i + 2 * k + 1] * b.v[6 * k + 2 * j + 1];
+						im += a.v[6 * i + 2 * k] * b.v[6 * k + 2 * j + 1] + a.v[6 * i + 2 * k + 1] * b.v[6 * k + 2 * j];
+					}
+					r.v[6 * i + 2 * j] = re;
+					r.v[6 * i + 2 * j + 1] = im;
+				}
+			complete_row2(r);
 			return r;
 		}
+	}
+	// c = a * b^dagger:  c_ij = sum_k a_ik conj(b_jk)
+	MESH_HD static E mul_nd_pairs(E const &a, E const &b)
+	{
+		E r;
 #pragma unroll
 		for (int i = 0; i < 3; ++i)
 #pragma unroll
@@ -410,6 +427,13 @@ template <class T> struct Group<SU3, T>
 				{
 					T ar = a.v[6 * i + 2 * k], ai = a.v[6 * i + 2 * k + 1];
 					T br = b.v[6 * j + 2 * k], bi = b.v[6 * j + 2 * k + 1];
+					// the first pair is the sum itself: 0 + x is x but for the sign of zero
+					if (sizeof(T) == 8 && k == 0)
+					{
+						re = ar * br + ai * bi;
+						im = ai * br - ar * bi;
+						continue;
+					}
 					re += ar * br + ai * bi;
 					im += ai * br - ar * bi;
 				}
@@ -417,6 +441,17 @@ template <class T> struct Group<SU3, T>
 				r.v[6 * i + 2 * j + 1] = im;
 			}
 		return r;
+	}
+	MESH_HD static E mul_nd(E const &a, E const &b)
+	{
+		if constexpr (kChain)
+		{
+			E r;
+			chain<3, false>(r, [&](int i, int k) { return a.at(i, k); }, [&](int k, int j) { return cconj(b.at(j, k)); });
+			return r;
+		}
+		else
+			return mul_nd_pairs(a, b);
 	}
 	// c = a^dagger * b:  c_ij = sum_k conj(a_ki) b_kj
 	MESH_HD static E mul_dn(E const &a, E const &b)
@@ -427,24 +462,27 @@ template <class T> struct Group<SU3, T>
 			chain<3, false>(r, [&](int i, int k) { return cconj(a.at(k, i)); }, [&](int k, int j) { return b.at(k, j); });
 			return r;
 		}
+		else
+		{
 #pragma unroll
-		for (int i = 0; i < 3; ++i)
+			for (int i = 0; i < 3; ++i)
 #pragma unroll
-			for (int j = 0; j < 3; ++j)
-			{
-				T re = 0, im = 0;
-#pragma unroll
-				for (int k = 0; k < 3; ++k)
+				for (int j = 0; j < 3; ++j)
 				{
-					T ar = a.v[6 * k + 2 * i], ai = a.v[6 * k + 2 * i + 1];
-					T br = b.v[6 * k + 2 * j], bi = b.v[6 * k + 2 * j + 1];
-					re += ar * br + ai * bi;
-					im += ar * bi - ai * br;
+					T re = 0, im = 0;
+#pragma unroll
+					for (int k = 0; k < 3; ++k)
+					{
+						T ar = a.v[6 * k + 2 * i], ai = a.v[6 * k + 2 * i + 1];
+						T br = b.v[6 * k + 2 * j], bi = b.v[6 * k + 2 * j + 1];
+						re += ar * br + ai * bi;
+						im += ar * bi - ai * br;
+					}
+					r.v[6 * i + 2 * j] = re;
+					r.v[6 * i + 2 * j + 1] = im;
 				}
-				r.v[6 * i + 2 * j] = re;
-				r.v[6 * i + 2 * j + 1] = im;
-			}
-		return r;
+			return r;
+		}
 	}
 	MESH_HD static E adj(E const &a)
 	{
@@ -805,21 +843,31 @@ template <class T> struct Group<SU3, T>
 		r.set(1, 2, cmul2(u1, b12, u2, q12));
 		return r;
 	}
-	// exp(t X) for X = from_alg(o) (antihermitian traceless), Cayley-Hamilton
+	// exp(t X) for X = from_alg(o) (antihermitian traceless): in FP64 the series for
+	// |tX| < 1, else exp_alg_closed
 	MESH_HD static E exp_alg(T const *o, T t)
 	{
-		T x[8];
-#pragma unroll
-		for (int k = 0; k < 8; ++k)
-			x[k] = o[k] * t;
 		if constexpr (sizeof(T) == 8)
 		{
+			T x[8];
+#pragma unroll
+			for (int k = 0; k < 8; ++k)
+				x[k] = o[k] * t;
 			T n01 = fma(x[2], x[2], x[3] * x[3]), n02 = fma(x[4], x[4], x[5] * x[5]);
 			T n12 = fma(x[6], x[6], x[7] * x[7]), a2 = x[0] + x[1];
 			T h = fma(T(0.5), fma(x[0], x[0], fma(x[1], x[1], a2 * a2)), n01 + n02 + n12);
 			if (h < T(0.5))
 				return exp_series_packed(x, n01, n02, n12, h);
 		}
+		return exp_alg_closed(o, t);
+	}
+	// the same by Cayley-Hamilton, in closed form (FP64) or for |tX| >= 1 (FP32)
+	MESH_HD static E exp_alg_closed(T const *o, T t)
+	{
+		T x[8];
+#pragma unroll
+		for (int k = 0; k < 8; ++k)
+			x[k] = o[k] * t;
 		E X = from_alg(x);
 		E X2 = sq_ah(X);
 		// c1 = Tr(Q^2)/2 = |X|^2/2,  c0 = det(Q) = det(-iX) = -Im det(X)
@@ -834,6 +882,17 @@ template <class T> struct Group<SU3, T>
 				return exp_series<10>(X, X2, c1, -c0);
 		}
 		cx<T> f0, f1, f2;
+		T const tiny = sizeof(T) == 8 ? T(1e-11) : T(1e-5);
+		if (c1 < tiny)
+		{
+			// exp(X) = 1 + X + X^2/2 + X^3/6; with X^3 = -i Q^3 and
+			// Q^3 = c1 Q + c0: 1 + X + X^2/2 - i (c1 Q + c0)/6
+			// -> f0 = 1 - i c0/6, f1 (on Q) = i - i c1/6, f2 (on Q^2) = -1/2
+			f0 = {T(1), -c0 * T(1.0 / 6.0)};
+			f1 = {T(0), T(1) - c1 * T(1.0 / 6.0)};
+			f2 = {T(-0.5), T(0)};
+		}
+		else
 		{
 			bool neg = c0 < T(0);
 			T c0a = neg ? -c0 : c0;

@@ -1728,7 +1728,7 @@ template <class T> __device__ __forceinline__ void or_power(T *h, T w)
 	T r0 = T(1) + w * a + c * (a * a - v2);
 	T f = w + T(2) * c * a;
 	T r1 = h[1] * f, r2 = h[2] * f, r3 = h[3] * f;
-	T n = m_rsqrt(r0 * r0 + r1 * r1 + r2 * r2 + r3 * r3);
+	T n = m_rsqrt_fast(r0 * r0 + r1 * r1 + r2 * r2 + r3 * r3);
 	h[0] = r0 * n;
 	h[1] = r1 * n;
 	h[2] = r2 * n;
@@ -1759,7 +1759,7 @@ template <class T> struct OrUpdate<SU2, T>
 		T n2 = W.v[0] * W.v[0] + W.v[1] * W.v[1] + W.v[2] * W.v[2] + W.v[3] * W.v[3];
 		if (n2 < T(1e-60))
 			return gx;
-		T n = m_rsqrt(n2);
+		T n = m_rsqrt_fast(n2);
 		T h[4] = {W.v[0] * n, -W.v[1] * n, -W.v[2] * n, -W.v[3] * n};
 		or_power(h, w);
 		E he = {{h[0], h[1], h[2], h[3]}};
@@ -1783,7 +1783,7 @@ template <class T> struct OrUpdate<SU3, T>
 			T n2 = q[0] * q[0] + q[1] * q[1] + q[2] * q[2] + q[3] * q[3];
 			if (n2 < T(1e-60))
 				continue;
-			T n = m_rsqrt(n2);
+			T n = m_rsqrt_fast(n2);
 			T h[4] = {q[0] * n, -q[1] * n, -q[2] * n, -q[3] * n};
 			or_power(h, w);
 			cx<T> a = {h[0], h[3]}, b = {h[2], h[1]}, c = {-h[2], h[1]}, d = {h[0], -h[3]};

@@ -24,8 +24,12 @@ template <int GRP, int ND> struct FaOps
 	{
 		auto &c = *U.ctx;
 		int64_t n = int64_t(ND) * U.geom.V;
-		k_fa_links<GRP, double, ND><<<grid_for(c, n, 256), 256, 0, c.stream>>>(
-		    U.geom, static_cast<double const *>(U.d), static_cast<double const *>(g.d), A, func);
+		auto const *u = static_cast<double const *>(U.d), *gd = static_cast<double const *>(g.d);
+		if (func.result) // its partial sums bound the grid
+			k_fa_links<GRP, double, ND, true><<<grid_for(c, n, kFaBlock, 16), kFaBlock, 0, c.stream>>>(U.geom, u, gd, A, func);
+		else
+			k_fa_links<GRP, double, ND, false>
+			    <<<unsigned((n + kFaBlock - 1) / kFaBlock), kFaBlock, 0, c.stream>>>(U.geom, u, gd, A, func);
 		MESH_LAUNCH_CHECK();
 	}
 	static void div(Field const &U, double const *A, float2 *buf, RedSlot theta)
@@ -38,7 +42,7 @@ template <int GRP, int ND> struct FaOps
 	static void update(Field const &U, float2 const *buf, Field const &gin, double *gout)
 	{
 		auto &c = *U.ctx;
-		k_fa_update<GRP, double, ND><<<grid_for(c, U.geom.V, 256), 256, 0, c.stream>>>(
+		k_fa_update<GRP, double, ND><<<unsigned((U.geom.V + kFaBlock - 1) / kFaBlock), kFaBlock, 0, c.stream>>>(
 		    U.geom, buf, static_cast<double const *>(gin.d), gout, 1.0 / double(U.geom.V));
 		MESH_LAUNCH_CHECK();
 	}

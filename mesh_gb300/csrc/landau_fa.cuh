@@ -73,9 +73,40 @@ __device__ __forceinline__ float mult_of(Multiplier const &m, MomTables const &m
 	return expf(m.table[i] * (1.f - f) + m.table[i + 1] * f);
 }
 
+// threads a block of the FP64 kernels below, a block for each 64 items: they are
+// bound by the FP64 pipe, so the SMs need equal shares. Blocks of 256 walked by
+// eight per SM gave 24^4 1296 blocks of work for 1216: some did twice the others'.
+// 24^4 SU(3) on a GB300: the links took 806 us, 792 in such blocks, 677
+// without the sum of the functional and the first adds of zero; the update 404 us
+constexpr int kFaBlock = 64;
+
+// products and exponential whose roundings the steps keep (Group<SU3, T>::kChain)
+template <int GRP, class T, class E> __device__ __forceinline__ E fa_mul(E const &a, E const &b)
+{
+	if constexpr (GRP == SU3)
+		return Group<GRP, T>::mul_pairs(a, b);
+	else
+		return Group<GRP, T>::mul(a, b);
+}
+template <int GRP, class T, class E> __device__ __forceinline__ E fa_mul_nd(E const &a, E const &b)
+{
+	if constexpr (GRP == SU3)
+		return Group<GRP, T>::mul_nd_pairs(a, b);
+	else
+		return Group<GRP, T>::mul_nd(a, b);
+}
+template <int GRP, class T> __device__ __forceinline__ typename Group<GRP, T>::E fa_exp(T const *o, T t)
+{
+	if constexpr (GRP == SU3)
+		return Group<GRP, T>::exp_alg_closed(o, t);
+	else
+		return Group<GRP, T>::exp_alg(o, t);
+}
+
 // A_mu(x) for every link, packed algebra, SoA per direction
-template <int GRP, class T, int ND>
-__global__ void __launch_bounds__(256) k_fa_links(Geom g, T const *__restrict__ U, T const *__restrict__ G,
+// (FUNC: with the sum of the functional, whose real parts are not formed otherwise)
+template <int GRP, class T, int ND, bool FUNC>
+__global__ void __launch_bounds__(kFaBlock) k_fa_links(Geom g, T const *__restrict__ U, T const *__restrict__ G,
                                                    T *__restrict__ A, RedSlot func)
 {
 	double acc = 0.0;
@@ -92,14 +123,14 @@ __global__ void __launch_bounds__(256) k_fa_links(Geom g, T const *__restrict__ 
 		Soa<T, Gp::NR>::load(G, g.V, s, gx.v);
 		Soa<T, Gp::NR>::load(G, g.V, eo_shift1<ND>(g, st, mu, +1), gf.v);
 		T a[Gp::NA];
-		E w = Gp::mul_nd(Gp::mul(gx, ld(mu, s)), gf);
-		if (func.result)
+		E w = fa_mul_nd<GRP, T>(fa_mul<GRP, T>(gx, ld(mu, s)), gf);
+		if constexpr (FUNC)
 			acc += double(Gp::retr(w));
 		Gp::proj(w, a);
 		comp<T, Gp::NA>(A, g.V, mu).store(s, a);
 	}
-	if (func.result) // uniform over the grid (a kernel argument)
-		grid_sum<256>(acc, func);
+	if constexpr (FUNC)
+		grid_sum<kFaBlock>(acc, func);
 }
 
 // Delta(x), theta sum, and the FP32 complex FFT input (lexicographic order)
@@ -159,7 +190,7 @@ __global__ void __launch_bounds__(256) k_fa_scale(float2 *__restrict__ buf, int6
 
 // g_out(x) = reunit(exp(-X(x)/V) g_in(x)), X from the transformed buffer
 template <int GRP, class T, int ND>
-__global__ void __launch_bounds__(256) k_fa_update(Geom g, float2 const *__restrict__ buf, T const *__restrict__ Gin,
+__global__ void __launch_bounds__(kFaBlock) k_fa_update(Geom g, float2 const *__restrict__ buf, T const *__restrict__ Gin,
                                                     T *__restrict__ Gout, T scale)
 {
 	using Gp = Group<GRP, T>;
@@ -179,7 +210,7 @@ __global__ void __launch_bounds__(256) k_fa_update(Geom g, float2 const *__restr
 		}
 		E gx;
 		Soa<T, Gp::NR>::load(Gin, g.V, s, gx.v);
-		E r = Gp::reunit_exact(Gp::mul(Gp::exp_alg(X, -scale), gx));
+		E r = Gp::reunit_exact(fa_mul<GRP, T>(fa_exp<GRP, T>(X, -scale), gx));
 		Soa<T, Gp::NR>::store(Gout, g.V, s, r.v);
 	}
 }
