@@ -86,6 +86,14 @@ double read_slot(Context &c, int k)
 	return v;
 }
 
+// the results of SLOT_TMP and SLOT_TMP2 in one transfer and wait
+void read_slots(Context &c, double *v)
+{
+	static_assert(SLOT_TMP2 == SLOT_TMP + 1, "adjacent slots");
+	MESH_CUDA(cudaMemcpyAsync(v, c.d_results + SLOT_TMP, 2 * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
+	MESH_CUDA(cudaStreamSynchronize(c.stream));
+}
+
 void create_field(Context &c, int kind, int group, int prec, int nd, int32_t const *dims, int nstack, Field &f)
 {
 	require(kind == MESH_GROUP || kind == MESH_ALGEBRA, "kind must be MESH_GROUP or MESH_ALGEBRA");
@@ -276,6 +284,19 @@ struct Workspace
 	Workspace(Workspace const &) = delete;
 	Workspace &operator=(Workspace const &) = delete;
 };
+
+// a single-component field on U's lattice in memory `d` that it does not own
+Field site_field(Field const &U, int kind, void *d)
+{
+	Field f = U;
+	f.kind = kind;
+	f.nstack = 1;
+	f.nr = kind == MESH_GROUP ? group_nr(U.group) : group_na(U.group);
+	f.bytes = size_t(U.geom.V) * size_t(f.nr) * f.real_bytes;
+	f.d = d;
+	return f;
+}
+size_t site_bytes_aligned(Field const &U, int kind) { return (site_field(U, kind, nullptr).bytes + 255) / 256 * 256; }
 
 // scratch for the momentum step on U's lattice from the context's workspace. Empty
 // (the step then runs without it) while the stream is being captured, as a later
@@ -1449,27 +1470,32 @@ static double landau_line_search(Field const &U, Field const &g, Field const &Fd
 	Context &c = *U.ctx;
 	auto const &ops = ops_for(U);
 	double norm_fac = 1.0 / (double(group_nc(U.group)) * U.nd * double(U.geom.V));
-	auto functional = [&](Field const &h) {
-		ops.landau_functional(U, h, slot(c, SLOT_TMP));
-		return read_slot(c, SLOT_TMP) * norm_fac;
+	// the functional at h into slot k; the results of two are read together (a
+	// read costs a wait for the stream, as long as the kernels of a small lattice)
+	auto functional = [&](Field const &h, int k) { ops.landau_functional(U, h, slot(c, k)); };
+	auto stepped = [&](double e, int k) {
+		ops.exp_apply(gt, Fd, e, g, false);
+		functional(gt, k);
 	};
-	auto stepped = [&](double e) {
-		ops.exp_apply(gt, Fd, e, g);
-		return functional(gt);
-	};
-	double base = functional(g);
-	double y1 = stepped(eps);
+	double y[2];
+	functional(g, SLOT_TMP);
+	stepped(eps, SLOT_TMP2);
+	read_slots(c, y);
+	double base = y[0] * norm_fac, y1 = y[1] * norm_fac;
 	while (y1 <= base)
 	{
 		eps *= 0.5;
-		y1 = stepped(eps);
+		stepped(eps, SLOT_TMP);
+		y1 = read_slot(c, SLOT_TMP) * norm_fac;
 		if (eps < 1e-10)
 			return 0.0;
 	}
-	double y2 = stepped(eps * 1.2);
+	stepped(eps * 1.2, SLOT_TMP);
+	stepped(eps * 0.8, SLOT_TMP2);
+	read_slots(c, y);
+	double y2 = y[0] * norm_fac, y3 = y[1] * norm_fac;
 	if (y2 > y1)
 		return 1.2 * eps;
-	double y3 = stepped(eps * 0.8);
 	double x1 = eps, x2 = 1.2 * eps, x3 = 0.8 * eps;
 	return 0.5 * ((x2 * x2 - x3 * x3) * y1 - (x1 * x1 - x3 * x3) * y2 + (x1 * x1 - x2 * x2) * y3) /
 	       ((x2 - x3) * y1 - (x1 - x3) * y2 + (x1 - x2) * y3);
@@ -1485,13 +1511,8 @@ int mesh_landau_line_search(mesh_field Uh, mesh_field gh, mesh_field Fh, double 
 		require(step != nullptr && eps > 0, "invalid argument");
 		Context &c = *U.ctx;
 		DeviceGuard dg(c.device);
-		Field gt;
-		struct Cleanup
-		{
-			Field *a;
-			~Cleanup() { destroy_field(*a); }
-		} cleanup{&gt};
-		create_field(c, MESH_GROUP, U.group, U.prec, U.nd, U.dims, 1, gt);
+		Workspace ws(c, site_bytes_aligned(U, MESH_GROUP));
+		Field gt = site_field(U, MESH_GROUP, ws.d);
 		*step = landau_line_search(U, g, Fd, gt, eps);
 	});
 }
@@ -1505,20 +1526,12 @@ int mesh_landau_cg(mesh_field Uh, mesh_field gh, int max_iter, double tol, int *
 		Context &c = *U.ctx;
 		DeviceGuard dg(c.device);
 		auto const &ops = ops_for(U);
-		Field Fd, last, gt;
-		struct Cleanup
-		{
-			Field *a, *b, *cc;
-			~Cleanup()
-			{
-				destroy_field(*a);
-				destroy_field(*b);
-				destroy_field(*cc);
-			}
-		} cleanup{&Fd, &last, &gt};
-		create_field(c, MESH_ALGEBRA, U.group, U.prec, U.nd, U.dims, 1, Fd);
-		create_field(c, MESH_ALGEBRA, U.group, U.prec, U.nd, U.dims, 1, last);
-		create_field(c, MESH_GROUP, U.group, U.prec, U.nd, U.dims, 1, gt);
+		// F, the last F and exp(eps F) g in the context's workspace
+		size_t na = site_bytes_aligned(U, MESH_ALGEBRA), nr = site_bytes_aligned(U, MESH_GROUP);
+		Workspace ws(c, 2 * na + nr);
+		char *w = static_cast<char *>(ws.d);
+		Field Fd = site_field(U, MESH_ALGEBRA, w), last = site_field(U, MESH_ALGEBRA, w + na),
+		      gt = site_field(U, MESH_GROUP, w + 2 * na);
 		MESH_CUDA(cudaMemsetAsync(last.d, 0, last.bytes, c.stream));
 		double norm_fac = 1.0 / (double(group_nc(U.group)) * U.nd * double(U.geom.V));
 		double eps = 3000.0, lastNorm = 0.0, th = 0.0;
@@ -1526,27 +1539,30 @@ int mesh_landau_cg(mesh_field Uh, mesh_field gh, int max_iter, double tol, int *
 		bool converged = false;
 		for (; it < max_iter; ++it)
 		{
-			th = landau_theta(U, g);
+			// theta, the derivative and its product with the last one, read together;
+			// F = -Delta norm_fac / 2, so <F, F> follows from theta's sum
+			double v[2], scale = -0.5 * norm_fac;
+			ops.landau_delta(Fd, U, g, scale, slot(c, SLOT_TMP));
+			ops.alg_dot(Fd, last, slot(c, SLOT_TMP2));
+			read_slots(c, v);
+			th = v[0] / (double(U.nd) * double(U.geom.V));
+			if (!std::isfinite(th))
+				throw Error(MESH_ERR_NUMERIC, "non-finite gauge condition theta");
 			if (th < tol)
 			{
 				converged = true;
 				break;
 			}
-			ops.landau_deriv(Fd, U, g, -0.5 * norm_fac);
 			// sum_real_trace(F*F) = -<F,F>, sum_real_trace(F*last) = -<F,last>
-			ops.alg_dot(Fd, Fd, slot(c, SLOT_TMP));
-			double norm = -read_slot(c, SLOT_TMP);
-			ops.alg_dot(Fd, last, slot(c, SLOT_TMP));
-			double fl = -read_slot(c, SLOT_TMP);
+			double norm = -scale * scale * v[0];
+			double fl = -v[1];
 			double beta = (norm - fl) / lastNorm;
 			MESH_CUDA(cudaMemcpyAsync(last.d, Fd.d, Fd.bytes, cudaMemcpyDeviceToDevice, c.stream));
 			// landau.h:126-128: `last = F; F += last * beta` (last already equals F)
 			if (it > 20 && beta > 0)
 				ops.axpy_alg(Fd, beta, last);
 			eps = landau_line_search(U, g, Fd, gt, eps);
-			ops.exp_apply(gt, Fd, eps, g);
-			MESH_CUDA(cudaMemcpyAsync(g.d, gt.d, g.bytes, cudaMemcpyDeviceToDevice, c.stream));
-			ops.reunitize(g);
+			ops.exp_apply(g, Fd, eps, g, true);
 			lastNorm = norm;
 		}
 		if (!converged)

@@ -72,7 +72,7 @@ enum SiteOp
 enum SlotId
 {
 	SLOT_TMP = 0,
-	SLOT_TMP2 = 1,
+	SLOT_TMP2 = 1, // follows SLOT_TMP: both results in one read
 };
 
 // device memory for the products of a momentum step (md_products.cuh): owned by
@@ -109,10 +109,12 @@ struct OpsTable
 	void (*landau_functional)(Field const &U, Field const &g, RedSlot out);
 	void (*landau_theta)(Field const &U, Field const &g, RedSlot out);
 	void (*landau_deriv)(Field &F, Field const &U, Field const &g, double scale);
+	// both in one pass: F and the sum of theta
+	void (*landau_delta)(Field &F, Field const &U, Field const &g, double scale, RedSlot out);
 	void (*landau_or_half)(Field const &U, Field &g, double omega, int parity);
 	void (*reunit_exact)(Field &g);
 	void (*alg_dot)(Field const &a, Field const &b, RedSlot out);
-	void (*exp_apply)(Field &dst, Field const &F, double eps, Field const &g);
+	void (*exp_apply)(Field &dst, Field const &F, double eps, Field const &g, bool reunit);
 	void (*axpy_alg)(Field &y, double a, Field const &x);
 	void (*gauge_transform)(Field &U, Field const &g);
 	// the HMC trajectory's plaquette, link update, momentum step and tuning:

@@ -1855,10 +1855,9 @@ __global__ void __launch_bounds__(kBlock)
 	grid_sum<kBlock>(acc, out);
 }
 
-// dst(x) = exp(eps F(x)) g(x)
+// dst(x) = exp(eps F(x)) g(x), with `reunit` projected on the group; dst may be g
 template <int GRP, class T>
-__global__ void __launch_bounds__(kBlock)
-    k_exp_apply(int64_t V, T eps, T const *__restrict__ F, T const *__restrict__ G, T *__restrict__ dst)
+__global__ void __launch_bounds__(kBlock) k_exp_apply(int64_t V, T eps, T const *__restrict__ F, T const *G, T *dst, int reunit)
 {
 	using Gp = Group<GRP, T>;
 	using E = typename Gp::E;
@@ -1869,6 +1868,8 @@ __global__ void __launch_bounds__(kBlock)
 		E gx;
 		Soa<T, Gp::NR>::load(G, V, s, gx.v);
 		E r = Gp::mul(Gp::exp_alg(f, eps), gx);
+		if (reunit)
+			r = Gp::reunit_fast(r);
 		Soa<T, Gp::NR>::store(dst, V, s, r.v);
 	}
 }
@@ -2027,6 +2028,11 @@ template <int GRP, class T, int ND> struct Ops
 	// lattices (8^4 SU(3): 256 blocks of 64, where 64 blocks of 256 left 88 of 152
 	// SMs idle; momentum refresh 27.9 -> 17.9 us, link update 21.4 -> 12.9 us)
 	static constexpr int kElemBlock = sizeof(T) == 8 ? 64 : kBlock;
+	// a block for each kElemBlock items in FP64, FP32 kernels walk theirs
+	static unsigned elem_grid(Context const &c, int64_t n)
+	{
+		return sizeof(T) == 8 ? unsigned((n + kElemBlock - 1) / kElemBlock) : blocks(c, n);
+	}
 	static unsigned elem_blocks(Context const &c, int64_t n, int per_sm)
 	{
 		unsigned b = grid_for(c, n, kElemBlock, per_sm * (kBlock / kElemBlock));
@@ -2116,14 +2122,14 @@ template <int GRP, class T, int ND> struct Ops
 	{
 		auto &c = *U.ctx;
 		int64_t n = int64_t(U.nstack) * U.geom.V;
-		k_reunit<GRP, T, false><<<blocks(c, n), kBlock, 0, c.stream>>>(n, U.geom.V, static_cast<T *>(U.d));
+		k_reunit<GRP, T, false><<<elem_grid(c, n), kElemBlock, 0, c.stream>>>(n, U.geom.V, static_cast<T *>(U.d));
 		MESH_LAUNCH_CHECK();
 	}
 	static void reunit_exact(Field &U)
 	{
 		auto &c = *U.ctx;
 		int64_t n = int64_t(U.nstack) * U.geom.V;
-		k_reunit<GRP, T, true><<<blocks(c, n), kBlock, 0, c.stream>>>(n, U.geom.V, static_cast<T *>(U.d));
+		k_reunit<GRP, T, true><<<elem_grid(c, n), kElemBlock, 0, c.stream>>>(n, U.geom.V, static_cast<T *>(U.d));
 		MESH_LAUNCH_CHECK();
 	}
 	static void hmc_evolve(Field const &Usrc, Field &Udst, Field const &P, double t, bool reunit)
@@ -2150,11 +2156,11 @@ template <int GRP, class T, int ND> struct Ops
 		auto &c = *Udst.ctx;
 		int64_t n = int64_t(Udst.nstack) * Udst.geom.V;
 		if (reunit)
-			k_evolve<GRP, T, true><<<elem_blocks(c, n, 8), kElemBlock, 0, c.stream>>>(
+			k_evolve<GRP, T, true><<<elem_grid(c, n), kElemBlock, 0, c.stream>>>(
 			    n, Udst.geom.V, static_cast<T const *>(Usrc.d), static_cast<T *>(Udst.d),
 			    static_cast<T const *>(P.d), T(t));
 		else
-			k_evolve<GRP, T, false><<<elem_blocks(c, n, 8), kElemBlock, 0, c.stream>>>(
+			k_evolve<GRP, T, false><<<elem_grid(c, n), kElemBlock, 0, c.stream>>>(
 			    n, Udst.geom.V, static_cast<T const *>(Usrc.d), static_cast<T *>(Udst.d),
 			    static_cast<T const *>(P.d), T(t));
 		MESH_LAUNCH_CHECK();
@@ -2954,6 +2960,14 @@ template <int GRP, class T, int ND> struct Ops
 		    RedSlot{});
 		MESH_LAUNCH_CHECK();
 	}
+	// theta and the derivative from one pass
+	static void landau_delta(Field &F, Field const &U, Field const &g, double scale, RedSlot out)
+	{
+		auto &c = *U.ctx;
+		k_landau_delta<GRP, T, ND, true, true><<<red_site_blocks(c, U.geom.V), 32 * ND, 0, c.stream>>>(
+		    U.geom, static_cast<T const *>(U.d), static_cast<T const *>(g.d), static_cast<T *>(F.d), T(scale), out);
+		MESH_LAUNCH_CHECK();
+	}
 	static void landau_or_half(Field const &U, Field &g, double omega, int parity)
 	{
 		auto &c = *U.ctx;
@@ -2969,11 +2983,12 @@ template <int GRP, class T, int ND> struct Ops
 		                                                            static_cast<T const *>(b.d), out);
 		MESH_LAUNCH_CHECK();
 	}
-	static void exp_apply(Field &dst, Field const &F, double eps, Field const &g)
+	static void exp_apply(Field &dst, Field const &F, double eps, Field const &g, bool reunit)
 	{
 		auto &c = *g.ctx;
-		k_exp_apply<GRP, T><<<blocks(c, g.geom.V), kBlock, 0, c.stream>>>(
-		    g.geom.V, T(eps), static_cast<T const *>(F.d), static_cast<T const *>(g.d), static_cast<T *>(dst.d));
+		k_exp_apply<GRP, T><<<elem_grid(c, g.geom.V), kElemBlock, 0, c.stream>>>(
+		    g.geom.V, T(eps), static_cast<T const *>(F.d), static_cast<T const *>(g.d), static_cast<T *>(dst.d),
+		    reunit ? 1 : 0);
 		MESH_LAUNCH_CHECK();
 	}
 	static void axpy_alg(Field &y, double a, Field const &x)
@@ -3073,7 +3088,7 @@ template <int GRP, class T, int ND> struct Ops
 		static const OpsTable t = {import_,      export_,       set_unit,       random,  random_momenta_dev,       norm2,
 		                           cshift,       site_op,       sum_real_trace, plaquette,      staple_sum,
 		                           wilson_deriv, reunitize,     evolve,         momentum_step,  landau_functional,
-		                           landau_theta, landau_deriv,  landau_or_half, reunit_exact,   alg_dot,
+		                           landau_theta, landau_deriv,  landau_delta, landau_or_half, reunit_exact,   alg_dot,
 		                           exp_apply,    axpy_alg,      gauge_transform,
 		                           hmc_plaquette, hmc_evolve,   hmc_momentum_step,
 		                           hmc_md_step,   hmc_tune_md,  wilson_partials, temporal_lines, spatial_lines, wilson_t,
