@@ -195,8 +195,9 @@ int mesh_overrelax_sweep(mesh_field U);
  * (spatial line of r links, temporal line of t links, averaged over sites and
  * the three spatial directions), normalised like the plaquette (ReTr / Nc, so
  * W(1, 1) is the mean plaquette of the planes (mu, 3)). out[(r-1) max_t + t-1].
- * 4D lattices; max_r <= min(L0, L1, L2), max_t <= L3. Allocates (max_t + 3)
- * link components of scratch for the call. */
+ * 4D lattices; max_r <= min(L0, L1, L2), max_t <= L3. Uses (max_t + 3) link
+ * components of the context's workspace, which keeps up to 512 MB between calls
+ * (more is allocated for the call). */
 int mesh_wilson_loops(mesh_field U, int max_r, int max_t, double *out);
 
 /* Plaquette without any device allocation. No counterpart in the reference.
@@ -253,7 +254,10 @@ int mesh_make_deltas(const char *scheme, double epsilon, int substeps, double *o
  * Owns U, P and the proposal U_new. Momenta and the Metropolis uniform come
  * from counter-based device streams keyed by `seed` and the trajectory
  * number; H_old/H_new, dH and the accept decision are computed on the device
- * in FP64. */
+ * in FP64. SU(3) chains also own the scratch of a molecular-dynamics step (192
+ * bytes a site in FP32, 2112 in FP64, at most 256 MB, or two slices of dimension
+ * 0 where those are more); a chain made without the memory for it runs the
+ * kernels that need none. */
 typedef struct mesh_hmc_record
 {
 	double plaquette; /* plaquette(U) after the accept/reject step */
