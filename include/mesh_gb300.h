@@ -254,10 +254,10 @@ int mesh_make_deltas(const char *scheme, double epsilon, int substeps, double *o
  * Owns U, P and the proposal U_new. Momenta and the Metropolis uniform come
  * from counter-based device streams keyed by `seed` and the trajectory
  * number; H_old/H_new, dH and the accept decision are computed on the device
- * in FP64. SU(3) chains also own the scratch of a molecular-dynamics step (192
- * bytes a site in FP32, 2112 in FP64, at most 256 MB, or two slices of dimension
- * 0 where those are more); a chain made without the memory for it runs the
- * kernels that need none. */
+ * in FP64. The SU(3) chains of a context share the scratch of a
+ * molecular-dynamics step (192 bytes a site in FP32, 2112 in FP64, of the largest
+ * chain, at most 256 MB, or two slices of dimension 0 where those are more); a
+ * chain made without the memory for it runs the kernels that need none. */
 typedef struct mesh_hmc_record
 {
 	double plaquette; /* plaquette(U) after the accept/reject step */

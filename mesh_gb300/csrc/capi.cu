@@ -42,6 +42,7 @@ void teardown_ctx(Context &c)
 		cudaFree(c.d_stage);
 	if (c.d_work)
 		cudaFree(c.d_work);
+	c.md_shared.reset();
 	if (c.own_stream && c.stream)
 		cudaStreamDestroy(c.stream);
 }
@@ -355,6 +356,7 @@ struct mesh_hmc_s
 	bool S_valid = false;
 	// products or plaquettes of a momentum step
 	MdScratch scratch;
+	std::shared_ptr<void> scratch_mem;
 	// cached CUDA graph of one trajectory
 	cudaGraphExec_t graph = nullptr;
 	double graph_beta = 0;
@@ -400,19 +402,26 @@ struct mesh_hmc_s
 		drop_graph();
 	}
 
-	// the chain's scratch; a chain without the memory for it steps without it
+	// the chain's share of the context's scratch; a chain made without the memory
+	// for it steps without it
 	void make_scratch()
 	{
 		size_t need = ops_for(U.f).md_scratch_bytes(U.f.geom, true);
 		if (need == 0)
 			return;
-		if (cudaMalloc(&scratch.d, need) == cudaSuccess)
-			scratch.bytes = need;
-		else
+		if (ctx->md_shared_bytes < need)
 		{
-			cudaGetLastError();
-			scratch.d = nullptr;
+			void *d = nullptr;
+			if (cudaMalloc(&d, need) != cudaSuccess)
+			{
+				cudaGetLastError();
+				return;
+			}
+			ctx->md_shared = std::shared_ptr<void>(d, [](void *p) { cudaFree(p); });
+			ctx->md_shared_bytes = need;
 		}
+		scratch_mem = ctx->md_shared;
+		scratch = {scratch_mem.get(), ctx->md_shared_bytes};
 	}
 
 	// Enqueue one trajectory (runHmcUpdate, hmc.cpp:73-107) on the stream.
@@ -1137,7 +1146,7 @@ int mesh_hmc_destroy(mesh_hmc h)
 		cudaFree(h->d_hist);
 		cudaFree(h->d_flag);
 		cudaFree(h->d_part);
-		cudaFree(h->scratch.d);
+		h->scratch_mem.reset();
 		cudaFree(h->d_res);
 		cudaFree(h->d_cnt);
 		// the fields hold the chain's references to the context

@@ -6,6 +6,7 @@
 
 #include <cstdint>
 #include <cstdio>
+#include <memory>
 #include <stdexcept>
 #include <string>
 
@@ -89,6 +90,13 @@ struct Context
 		work_bytes = bytes;
 		return true;
 	}
+
+	// scratch of the chains' molecular-dynamics steps, one for all chains of the
+	// context: they run on its stream one after another and nothing stays in it
+	// between steps. A chain keeps the memory it was made with (its captured
+	// trajectory holds the address); a larger chain replaces what later ones share.
+	std::shared_ptr<void> md_shared;
+	size_t md_shared_bytes = 0;
 
 	void *stage(size_t bytes)
 	{

@@ -75,8 +75,8 @@ enum SlotId
 	SLOT_TMP2 = 1, // follows SLOT_TMP: both results in one read
 };
 
-// device memory for the products of a momentum step (md_products.cuh): owned by
-// a chain (a captured trajectory holds its address) or by a context
+// device memory for the products or plaquettes of a momentum step: shared by a
+// context's chains (a captured trajectory holds its address) or its workspace
 struct MdScratch
 {
 	void *d = nullptr;

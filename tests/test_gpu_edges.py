@@ -168,3 +168,41 @@ def test_run_hmd_fused_steps(ctx, oracle, g, p, dims, steps):
     Uo, Po = oracle.run_hmd(g, 2, dims, U64, P64, 2.0 * g, d)
     tol = 1e-12 if p == 2 else 2e-5
     assert rel(U.export(), Uo) < tol and rel(P.export(), Po) < tol
+
+
+@pytest.mark.parametrize("p", [1, 2])
+def test_chains_share_step_scratch(p):
+    """graph-replayed chains of a context in turn, the second larger (its scratch
+    replaces what later chains share), the third made after the first is gone:
+    each as on a context of its own"""
+    shapes, d = [[4, 4, 6, 4], [8, 6, 4, 10], [4, 6, 4, 4]], mg.make_deltas("2lf", 0.5, 4)
+
+    def chain(ctx, k):
+        h = mg.Hmc(ctx, 3, p, mg.Grid(shapes[k]), seed=5 + k)
+        h.cold_start()
+        return h
+
+    alone = []
+    for k in range(3):
+        c = mg.Context(0)
+        h = chain(c, k)
+        h.run(5.7, d, 3)
+        alone.append((h.U.export(), h.history()["plaq_history"]))
+        h.close()
+        c.close()
+    c = mg.Context(0)
+    a = chain(c, 0)
+    a.run(5.7, d, 1)
+    b = chain(c, 1)
+    for _ in range(2):
+        b.run(5.7, d, 1)
+        a.run(5.7, d, 1)
+    got = [(a.U.export(), a.history()["plaq_history"])]
+    a.close()
+    e = chain(c, 2)
+    b.run(5.7, d, 1)
+    e.run(5.7, d, 3)
+    got += [(h.U.export(), h.history()["plaq_history"]) for h in (b, e)]
+    for (u, pl), (uo, plo) in zip(got, alone):
+        assert rel(u, uo) < (1e-12 if p == 2 else 2e-5)
+        assert rel(pl, plo) < (1e-12 if p == 2 else 1e-6)
