@@ -100,6 +100,11 @@ template <class T> struct Group<U1, T>
 	MESH_HD static E unit() { return {{T(1), T(0)}}; }
 	MESH_HD static E zero() { return {{T(0), T(0)}}; }
 	MESH_HD static E mul(E a, E b) { return {{a.v[0] * b.v[0] - a.v[1] * b.v[1], a.v[0] * b.v[1] + a.v[1] * b.v[0]}}; }
+	// c + a * b, the sum inside the products
+	MESH_HD static E mul_add(E c, E a, E b)
+	{
+		return {{fma(-a.v[1], b.v[1], fma(a.v[0], b.v[0], c.v[0])), fma(a.v[1], b.v[0], fma(a.v[0], b.v[1], c.v[1]))}};
+	}
 	// a * b^dagger
 	MESH_HD static E mul_nd(E a, E b) { return {{a.v[0] * b.v[0] + a.v[1] * b.v[1], a.v[1] * b.v[0] - a.v[0] * b.v[1]}}; }
 	// a^dagger * b
@@ -186,6 +191,14 @@ template <class T> struct Group<SU2, T>
 		         a.v[0] * b.v[3] + a.v[1] * b.v[2] - a.v[2] * b.v[1] + a.v[3] * b.v[0]}};
 	}
 	MESH_HD static E adj(E a) { return {{a.v[0], -a.v[1], -a.v[2], -a.v[3]}}; }
+	// c + a * b, the sum inside the products
+	MESH_HD static E mul_add(E c, E a, E b)
+	{
+		return {{fma(-a.v[3], b.v[3], fma(-a.v[2], b.v[2], fma(-a.v[1], b.v[1], fma(a.v[0], b.v[0], c.v[0])))),
+		         fma(-a.v[3], b.v[2], fma(a.v[2], b.v[3], fma(a.v[1], b.v[0], fma(a.v[0], b.v[1], c.v[1])))),
+		         fma(a.v[3], b.v[1], fma(a.v[2], b.v[0], fma(-a.v[1], b.v[3], fma(a.v[0], b.v[2], c.v[2])))),
+		         fma(a.v[3], b.v[0], fma(-a.v[2], b.v[1], fma(a.v[1], b.v[2], fma(a.v[0], b.v[3], c.v[3]))))}};
+	}
 	MESH_HD static E mul_nd(E a, E b) { return mul(a, adj(b)); }
 	MESH_HD static E mul_dn(E a, E b) { return mul(adj(a), b); }
 	MESH_HD static void add_to(E &a, E b)

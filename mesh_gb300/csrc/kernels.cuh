@@ -1597,6 +1597,29 @@ template <int GRP, class T, class E> __device__ __forceinline__ void add_closing
 		Gp::add_to(K, Gp::adj(Gp::mul(gb, ub)));
 	}
 }
+// the same less 2 g(x)^+, each product summed onto -g(x)^+ (the sign costs nothing)
+template <int GRP, class T, class E>
+__device__ __forceinline__ E closing_less_g(E const &u, E const &gf, E const &gb, E const &ub, E const &gx)
+{
+	using Gp = Group<GRP, T>;
+	E m = Gp::adj(gx);
+#pragma unroll
+	for (int r = 0; r < Gp::NR; ++r)
+		m.v[r] = -m.v[r];
+	E K = m, b = m;
+	if constexpr (GRP == SU3)
+	{
+		Gp::add_nd(K, u, gf);
+		Gp::add_mul_adj(b, gb, ub);
+	}
+	else
+	{
+		K = Gp::mul_add(m, u, Gp::adj(gf));
+		b = Gp::mul_add(m, Gp::adj(ub), Gp::adj(gb));
+	}
+	Gp::add_to(K, b);
+	return K;
+}
 
 // sum_x sum_mu ReTr(g(x) U_mu(x) g(x+mu)^+)
 template <int GRP, class T, int ND>
@@ -1641,7 +1664,8 @@ template <int GRP, class T, int ND> struct ClosingSum
 	T k[ND][Gp::NR][32];
 
 	// K of the block's 32 sites (valid: this lane's site exists); the result in
-	// warp 0 only. Every thread of the block must call it.
+	// warp 0 only. Every thread of the block must call it. LESS_G: K - 2 ND g(x)^+.
+	template <bool LESS_G = false>
 	__device__ __forceinline__ E sum(Geom const &g, bool valid, Site<ND> const &st, int64_t s,
 	                                 LinkLoad<GRP, T, ND> const &ld, T const *G)
 	{
@@ -1653,7 +1677,14 @@ template <int GRP, class T, int ND> struct ClosingSum
 			int64_t b = eo_shift1<ND>(g, st, mu, -1);
 			Soa<T, Gp::NR>::load(G, g.V, eo_shift1<ND>(g, st, mu, +1), gf.v);
 			Soa<T, Gp::NR>::load(G, g.V, b, gb.v);
-			add_closing<GRP, T>(K, ld(mu, s), gf, gb, ld(mu, b));
+			if constexpr (LESS_G)
+			{
+				E gx;
+				Soa<T, Gp::NR>::load(G, g.V, s, gx.v);
+				K = closing_less_g<GRP, T>(ld(mu, s), gf, gb, ld(mu, b), gx);
+			}
+			else
+				add_closing<GRP, T>(K, ld(mu, s), gf, gb, ld(mu, b));
 		}
 		if (mu > 0)
 		{
@@ -1679,8 +1710,14 @@ template <int GRP, class T, int ND> struct ClosingSum
 // Delta(x) = proj(g(x) K(x)) for any matrices: 9 products a site where the A_mu
 // one by one take 16. THETA: sum_x |Delta(x)|^2 into out; DERIV: F = scale
 // Delta (Landau::deriv, landau.h:52-65).
+// K enters less 2 ND g(x)^+, which leaves Delta as it is (g g^+ is hermitian): near
+// the gauge K is 2 ND g^+ and a small rest, and Delta is what proj leaves of it, so
+// rounded at the size of the whole K it added 3 to 9 times as much to theta as the
+// A_mu one by one (pure gauge SU(3) 4x4x6x8: 4.6e-14 against 0.7e-14 in FP32,
+// 1.6e-31 against 0.2e-31 in FP64); onto -g^+ each product rounds at the size of the
+// rest, and theta gets no more than from the A_mu.
 // 24^4 SU(3) FP64 on a GB300: theta took 1519 us from the A_mu with a thread per
-// site, 636 us here (1039 FP64 operations a site, the pipe 90% busy).
+// site, 636 us from the whole K, 662 here (1111 FP64 operations a site).
 template <int GRP, class T, int ND, bool THETA, bool DERIV>
 __global__ void __launch_bounds__(32 * ND)
     k_landau_delta(Geom g, T const *__restrict__ U, T const *__restrict__ G, T *__restrict__ F, T scale, RedSlot out)
@@ -1695,7 +1732,7 @@ __global__ void __launch_bounds__(32 * ND)
 		int64_t s = s0 + (threadIdx.x & 31);
 		bool valid = s < g.V;
 		Site<ND> st = site_from_eo<ND>(g, valid ? s : 0);
-		E K = sm.sum(g, valid, st, s, ld, G);
+		E K = sm.template sum<true>(g, valid, st, s, ld, G);
 		if (threadIdx.x < 32 && valid)
 		{
 			E gx;
