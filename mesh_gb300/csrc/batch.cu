@@ -378,7 +378,7 @@ __global__ void __launch_bounds__(kChunk, MB)
 	batch_loop<KIN, T>(sp, kin, [&](int r, BatchRep const &rep, int, int64_t s, Site<kBND> const &st) {
 		LinkLoad<GRP, T, kBND, kRows<GRP, T>> ld{static_cast<T const *>(flip ? rep.Ut : rep.Unew), rep.g.V};
 		T coef = T(beta[r] / (2.0 * Gp::NC) * dp);
-		double k = site_md<GRP, T, kBND, F2, kRows<GRP, T>, true, decltype(ld), false, false, GENERIC>(
+		double k = site_md<GRP, T, kBND, F2, kRows<GRP, T>, true, decltype(ld), false, false, GENERIC, false>(
 		    rep.g, st, s, ld, static_cast<T *>(rep.P), coef, static_cast<T *>(flip ? rep.Unew : rep.Ut), T(du),
 		    reunit, KIN);
 		return KIN ? T(k) : T(0); // k is the site's sum in T, exactly

@@ -796,7 +796,11 @@ template <int ND, int NA, class T> __device__ __forceinline__ void add_dir(T (&F
 // four dimensions: x + e_mu, x - e_nu, x - e_nu + e_mu) computed once per site
 // instead of once per staple: for these groups the products are a few FMAs, and the
 // index arithmetic, not the arithmetic of the staples, set the instruction count.
-template <int GRP, class T, int ND, bool FUSE, class LD>
+// FINE: the kinetic norm is summed link by link in FP64, as the kernels with a thread
+// per link and H_old sum it (in the field precision, four links to an FP64 add, dH of
+// unchanged FP32 momenta was off by up to 7e-9 of H). The batched replicas' kernel,
+// which spills registers, does without.
+template <int GRP, class T, int ND, bool FUSE, bool FINE, class LD>
 __device__ __forceinline__ double site_md_small(Geom const &g, Site<ND> const &st, int64_t s, LD const &ld,
                                                 T *__restrict__ P, T coef, T *__restrict__ Uout, T tu, int reunit,
                                                 bool want_kin)
@@ -860,7 +864,7 @@ __device__ __forceinline__ double site_md_small(Geom const &g, Site<ND> const &s
 		for (int a = 0; a < NA; ++a)
 			F[mu][a] += xa[a];
 	}
-	T kacc = T(0); // the site's kinetic terms in the field precision, one FP64 add per site
+	std::conditional_t<FINE, double, T> kacc = 0;
 #pragma unroll
 	for (int mu = 0; mu < ND; ++mu)
 	{
@@ -971,14 +975,14 @@ template <class T, int ND, int NA> struct SiteAcc<T, ND, NA, true>
 // momentum step of a trajectory asks for it). Shared by k_momentum_step_site
 // and the batched replicas.
 template <int GRP, class T, int ND, int F2, bool ROWS, bool FUSE, class LD, bool SM = false, bool PIPE = false,
-          bool GENERIC = false>
+          bool GENERIC = false, bool FINE = true>
 __device__ __forceinline__ double site_md(Geom const &g, Site<ND> const &st, int64_t s, LD const &ld,
                                           T *__restrict__ P, T coef, T *__restrict__ Uout, T tu, int reunit,
                                           bool want_kin, T *acc_sm = nullptr)
 {
 	// GENERIC: the rolled plane/staple loops below for every group
 	if constexpr (GRP != SU3 && ND == 4 && !SM && !PIPE && !GENERIC)
-		return site_md_small<GRP, T, ND, FUSE>(g, st, s, ld, P, coef, Uout, tu, reunit, want_kin);
+		return site_md_small<GRP, T, ND, FUSE, FINE>(g, st, s, ld, P, coef, Uout, tu, reunit, want_kin);
 	using Gp = Group<GRP, T>;
 	using E = typename Gp::E;
 	using Pr = Prod<GRP, T, F2>;
@@ -1249,7 +1253,7 @@ __global__ void __launch_bounds__(128)
 		if (!slab_site(g, g.V, 0, 1, tile, s))
 			continue;
 		Site<ND> st = site_from_eo<ND>(g, s);
-		double k = site_md_small<GRP, T, ND, FUSE>(g, st, s, ld, P, coef, Uout, tu, reunit, kin.result != nullptr);
+		double k = site_md_small<GRP, T, ND, FUSE, true>(g, st, s, ld, P, coef, Uout, tu, reunit, kin.result != nullptr);
 		if (kin.result)
 			acc += k;
 	}

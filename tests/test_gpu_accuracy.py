@@ -66,3 +66,20 @@ def test_landau_theta_in_the_gauge(ctx, oracle, g, p, dims):
                                                                      G.astype(np.float64)), rel=1e-6)
     plain = theta_per_link(g, dims, U, G, np.complex64 if p == 1 else np.complex128)
     assert abs(L.condition() - exact) <= 1.3 * abs(plain - exact)
+
+
+@pytest.mark.parametrize("variant", [-1, 58])
+@pytest.mark.parametrize("dims", [[6, 10], [64, 64], [6, 4, 10], [16, 24, 20], [2, 6, 4, 10], [6, 10, 14, 18]],
+                         ids=lambda d: "x".join(map(str, d)))
+@pytest.mark.parametrize("g,p", [(1, 1), (2, 1), (1, 2), (2, 2)])
+def test_kinetic_energy_of_unchanged_momenta(ctx, g, p, dims, variant):
+    """at beta = 0 the momenta stay and H is their norm: both ends of a trajectory sum
+    the same link terms in FP64 (some thousand additions: 1e-13)"""
+    h = mg.Hmc(ctx, g, p, mg.Grid(dims), seed=3)
+    P = mg.Momenta(ctx, g, p, mg.Grid(dims)).random(5)
+    try:
+        mg.force_variant(variant)
+        rec = h.update_supplied(P, 0.0, 0.0, [0.1, 0.2, 0.1])
+    finally:
+        mg.force_variant(-1)
+    assert abs(rec["H_new"] - rec["H_old"]) <= 1e-13 * rec["H_old"]
