@@ -100,6 +100,12 @@ template <class T> struct Group<U1, T>
 	MESH_HD static E unit() { return {{T(1), T(0)}}; }
 	MESH_HD static E zero() { return {{T(0), T(0)}}; }
 	MESH_HD static E mul(E a, E b) { return {{a.v[0] * b.v[0] - a.v[1] * b.v[1], a.v[0] * b.v[1] + a.v[1] * b.v[0]}}; }
+	// a * b for a near 1: the small terms first, so one rounding, not two, is of the
+	// size of b (which of the two mul has, the compiler chooses)
+	MESH_HD static E mul_near1(E a, E b)
+	{
+		return {{fma(a.v[0], b.v[0], -a.v[1] * b.v[1]), fma(a.v[0], b.v[1], a.v[1] * b.v[0])}};
+	}
 	// c + a * b, the sum inside the products
 	MESH_HD static E mul_add(E c, E a, E b)
 	{
@@ -191,6 +197,14 @@ template <class T> struct Group<SU2, T>
 		         a.v[0] * b.v[3] + a.v[1] * b.v[2] - a.v[2] * b.v[1] + a.v[3] * b.v[0]}};
 	}
 	MESH_HD static E adj(E a) { return {{a.v[0], -a.v[1], -a.v[2], -a.v[3]}}; }
+	// a * b for a near 1: the small terms first (see U(1))
+	MESH_HD static E mul_near1(E a, E b)
+	{
+		return {{fma(a.v[0], b.v[0], fma(-a.v[1], b.v[1], fma(-a.v[2], b.v[2], -a.v[3] * b.v[3]))),
+		         fma(a.v[0], b.v[1], fma(a.v[1], b.v[0], fma(a.v[2], b.v[3], -a.v[3] * b.v[2]))),
+		         fma(a.v[0], b.v[2], fma(-a.v[1], b.v[3], fma(a.v[2], b.v[0], a.v[3] * b.v[1]))),
+		         fma(a.v[0], b.v[3], fma(a.v[1], b.v[2], fma(-a.v[2], b.v[1], a.v[3] * b.v[0])))}};
+	}
 	// c + a * b, the sum inside the products
 	MESH_HD static E mul_add(E c, E a, E b)
 	{

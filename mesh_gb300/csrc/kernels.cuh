@@ -798,7 +798,10 @@ template <int ND, int NA, class T> __device__ __forceinline__ void add_dir(T (&F
 // index arithmetic, not the arithmetic of the staples, set the instruction count.
 // FINE: the kinetic norm is summed link by link in FP64, as the kernels with a thread
 // per link and H_old sum it (in the field precision, four links to an FP64 add, dH of
-// unchanged FP32 momenta was off by up to 7e-9 of H). The batched replicas' kernel,
+// unchanged FP32 momenta was off by up to 7e-9 of H), and the link update's product
+// rounds once at the size of the link (as it came out of mul, the links of FP32 U(1)
+// and SU(2) were 9% and 5% further from FP64's after ten steps than those of the
+// separate link update; now they are as close and 24% closer). The batched replicas' kernel,
 // which spills registers, does without.
 template <int GRP, class T, int ND, bool FUSE, bool FINE, class LD>
 __device__ __forceinline__ double site_md_small(Geom const &g, Site<ND> const &st, int64_t s, LD const &ld,
@@ -879,7 +882,11 @@ __device__ __forceinline__ double site_md_small(Geom const &g, Site<ND> const &s
 			kacc += Gp::kin(p);
 		if constexpr (FUSE)
 		{
-			E r = Gp::mul(Gp::exp_alg(p, tu), u[mu]);
+			E x = Gp::exp_alg(p, tu), r;
+			if constexpr (FINE)
+				r = Gp::mul_near1(x, u[mu]);
+			else
+				r = Gp::mul(x, u[mu]);
 			if (reunit)
 				r = Gp::reunit_fast(r);
 			comp<T, Gp::NR>(Uout, g.V, mu).store(s, r.v);
@@ -1238,8 +1245,10 @@ __global__ void __launch_bounds__(NT, MINB)
 // of 32 sites, even and odd ones in turn. A thread per link recomputes the index
 // arithmetic of every staple, which is most of its instructions for these groups.
 // U(1) FP32 64x96x80 on a GB300: momentum step 25.9 us a thread per link;
-// fused with the link update (7.6 us on its own) 16 us here.
-template <int GRP, class T, int ND, bool FUSE>
+// fused with the link update (7.6 us on its own) 13 us here.
+// KIN: with the kinetic norm, which a trajectory's last step asks for (asked at run
+// time, ten steps of that lattice took 177 us, without 136).
+template <int GRP, class T, int ND, bool FUSE, bool KIN>
 __global__ void __launch_bounds__(128)
     k_md_small(Geom g, T const *__restrict__ U, T *__restrict__ P, T coef, RedSlot kin, T *__restrict__ Uout, T tu,
                int reunit)
@@ -1253,11 +1262,11 @@ __global__ void __launch_bounds__(128)
 		if (!slab_site(g, g.V, 0, 1, tile, s))
 			continue;
 		Site<ND> st = site_from_eo<ND>(g, s);
-		double k = site_md_small<GRP, T, ND, FUSE, true>(g, st, s, ld, P, coef, Uout, tu, reunit, kin.result != nullptr);
-		if (kin.result)
+		double k = site_md_small<GRP, T, ND, FUSE, true>(g, st, s, ld, P, coef, Uout, tu, reunit, KIN);
+		if constexpr (KIN)
 			acc += k;
 	}
-	if (kin.result)
+	if constexpr (KIN)
 		grid_sum<128>(acc, kin);
 }
 
@@ -2401,7 +2410,7 @@ template <int GRP, class T, int ND> struct Ops
 	{
 		if constexpr (GRP != SU3)
 		{
-			auto k = k_md_small<GRP, T, ND, FUSE>;
+			auto k = kin.result ? k_md_small<GRP, T, ND, FUSE, true> : k_md_small<GRP, T, ND, FUSE, false>;
 			unsigned b = resident_grid(c, k, 128, (slab_tiles(g.V, 1) + 3) / 4);
 			k<<<b < unsigned(kMaxRedBlocks) ? b : unsigned(kMaxRedBlocks), 128, 0, c.stream>>>(g, u, p, coef, kin, uo, tu,
 			                                                                                 reunit);

@@ -83,3 +83,33 @@ def test_kinetic_energy_of_unchanged_momenta(ctx, g, p, dims, variant):
     finally:
         mg.force_variant(-1)
     assert abs(rec["H_new"] - rec["H_old"]) <= 1e-13 * rec["H_old"]
+
+
+@pytest.mark.parametrize("variant", [-1, 58])
+@pytest.mark.parametrize("dims", [[64, 64], [16, 24, 20], [6, 10, 14, 18], [16, 16, 8, 16]],
+                         ids=lambda d: "x".join(map(str, d)))
+@pytest.mark.parametrize("g", [1, 2])
+def test_fused_steps_round_no_more_than_separate_ones(ctx, g, dims, variant):
+    """ten leapfrog steps of FP32 links and momenta against the FP64 ones: the rms
+    distance of the fused steps at most 1.02 times that of momentum steps and link
+    updates apart (the 1.02: the spread of an rms over some thousand reals)"""
+    grid, beta, d = mg.Grid(dims), 2.0 * g, mg.make_deltas("2lf", 0.5, 10)
+
+    def fields(p, U=None, P=None):
+        u, m = mg.GaugeField(ctx, g, p, grid), mg.Momenta(ctx, g, p, grid)
+        return (u.random(3), m.random(5)) if U is None else (u.import_(U), m.import_(P))
+
+    U0, P0 = (f.export() for f in fields(mg.F32))
+    exact, fused, apart = fields(mg.F64, U0, P0), fields(mg.F32, U0, P0), fields(mg.F32, U0, P0)
+    try:
+        mg.force_variant(variant)
+        mg.run_hmd(*fused, beta, d)
+        mg.force_variant(0)
+        mg.run_hmd(*exact, beta, d)
+        for i, t in enumerate(d):
+            mg.momentum_step(apart[1], apart[0], beta, t) if i % 2 else mg.evolve(*apart, t)
+    finally:
+        mg.force_variant(-1)
+    for x, f, s in zip(exact, fused, apart):
+        ef, es = (np.sqrt(np.mean((y.export().astype(np.float64) - x.export()) ** 2)) for y in (f, s))
+        assert ef <= 1.02 * es, (ef, es)
