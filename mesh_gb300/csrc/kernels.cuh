@@ -725,36 +725,124 @@ template <int ND> __host__ __device__ constexpr int plane_nu(int q)
 	return mu + 1 + q;
 }
 
-// sum over sites and planes of the plaquette traces: tiles of 32 sites, one
-// warp per plane, walked by a grid of at most kPlaqBlocks<T> blocks per SM
-// (resident at once). A thread per site that loops over the planes bounds small
-// lattices by one thread's chain (8^4: 16 blocks on 152 SMs) and holds twice the
-// registers. SU(3) on a GB300, before and after: FP64 8^4 113 -> 32 us a call
+// ---- sum over sites and planes of the plaquette traces ------------------------
+// Two kernels. Tiles of 32 sites with one warp per plane (k_plaquette): a thread per
+// site bounds small lattices by one thread's chain over the planes and holds twice
+// the registers. SU(3) on a GB300, before and after: FP64 8^4 113 -> 32 us a call
 // (kernel 18), FP32 32^4 (rows 0, 1 read) 142 -> 128 us.
-template <class T> inline constexpr int kPlaqBlocks = sizeof(T) == 8 ? 2 : 4;
+// U(1) and SU(2) do a few operations a load and live on loads in flight: a thread per
+// site (k_plaquette_site) shares the site's links and index arithmetic between the
+// planes. FP32, tiles against sites: U(1) 48^4 275 -> 62 us, 128^3 49 -> 19, SU(2)
+// 48^4 296 -> 113, 128^3 121 -> 30, 12^3x24 8.4 -> 6.4 and 8.3, no size slower. In
+// FP64 the pipe (a warp's instruction every 16 cycles per SM) binds both on large
+// lattices and the tiles spread better over the SMs on small ones: U(1) 8^4 6.3 in
+// tiles against 8.4 by sites, 24^4 47 against 49, SU(2) 8^4 8.3 against 12.5, 24^4 135
+// against 139; 128^3 U(1) 199 against 133 and SU(2) 508 against 407, 48^4 U(1) 751
+// against 631. Sites from 2^19 on.
+constexpr int kPlaqThreads = 192;
+constexpr int kPlaqSiteThreads = 256;
 template <int ND> inline constexpr int kPlanes = ND * (ND - 1) / 2;
-template <class T> inline unsigned plaquette_grid(int num_sms, int64_t V)
+// blocks per SM, resident at once. FP32 tiles: four in four dimensions (SU(3) 32^4 160
+// us, 177 with two), two below, where 80 registers spill (128^3 173 us with four, 160)
+template <class T, int ND> inline constexpr int kPlaqBlocks = sizeof(T) == 4 && ND == 4 ? 4 : 2;
+template <class T> inline constexpr int kPlaqSiteBlocks = sizeof(T) == 4 ? 4 : 3;
+template <int GRP, class T> inline bool plaquette_by_site(int64_t V)
 {
-	int64_t tiles = (V + 31) / 32, cap = int64_t(num_sms) * kPlaqBlocks<T>;
-	return unsigned(tiles < cap ? tiles : cap);
+	return GRP != SU3 && (sizeof(T) == 4 || V >= int64_t(1) << 19);
 }
+template <int GRP, class T, int ND> inline unsigned plaquette_grid(int num_sms, int64_t V)
+{
+	bool site = plaquette_by_site<GRP, T>(V);
+	int64_t need = site ? (V + kPlaqSiteThreads - 1) / kPlaqSiteThreads : (V + 31) / 32;
+	int64_t cap = int64_t(num_sms) * (site ? kPlaqSiteBlocks<T> : kPlaqBlocks<T, ND>);
+	return unsigned(need < cap ? need : cap);
+}
+// A block holds the warps of 6 / planes tiles, gridDim.x tiles apart: a block for each
+// tile first (FP64 SU(3) 64^2: 12.5 us, 16.6 with six tiles to a block), and where the
+// tiles are more than the blocks every warp has one (254^2: 60 us with a block of one
+// warp for each tile at two per SM, 41 here)
 template <int GRP, class T, int ND, bool ROWS = false>
-__global__ void __launch_bounds__(32 * kPlanes<ND>, kPlaqBlocks<T>)
+__global__ void __launch_bounds__(kPlaqThreads, kPlaqBlocks<T, ND>)
     k_plaquette(Geom g, T const *__restrict__ U, RedSlot out)
 {
 	using Gp = Group<GRP, T>;
 	using E = typename Gp::E;
+	constexpr int kTiles = kPlaqThreads / 32 / kPlanes<ND>;
 	LinkLoad<GRP, T, ND, ROWS> ld{U, g.V};
-	int w = threadIdx.x >> 5, mu = plane_mu<ND>(w), nu = plane_nu<ND>(w);
+	int w = threadIdx.x >> 5, q = w % kPlanes<ND>, mu = plane_mu<ND>(q), nu = plane_nu<ND>(q);
+	int64_t step = int64_t(gridDim.x) * 32;
 	double acc = 0.0;
-	for (int64_t s = int64_t(blockIdx.x) * 32 + (threadIdx.x & 31); s < g.V; s += int64_t(gridDim.x) * 32)
+	for (int64_t s = int64_t(blockIdx.x) * 32 + (threadIdx.x & 31) + w / kPlanes<ND> * step; s < g.V; s += kTiles * step)
 	{
 		Site<ND> st = site_from_eo<ND>(g, s);
 		E ab = Gp::mul(ld(mu, s), ld(nu, eo_shift1<ND>(g, st, mu, +1)));
 		E dc = Gp::mul(ld(nu, s), ld(mu, eo_shift1<ND>(g, st, nu, +1)));
 		acc += double(Gp::retr_nd(ab, dc));
 	}
-	grid_sum<32 * kPlanes<ND>>(acc, out);
+	grid_sum<kPlaqThreads>(acc, out);
+}
+// a sum in two floats (Knuth's two-sum; Dekker 1971): as good as FP64 for a thread's
+// few thousand FP32 terms, without the FP64 pipe (an FP64 add for each plane takes
+// U(1) 32^4 from 17 to 33 us)
+template <class T> struct Sum
+{
+	double v = 0.0;
+	__device__ __forceinline__ void add(T x) { v += x; }
+	__device__ __forceinline__ double get() const { return v; }
+};
+template <> struct Sum<float>
+{
+	float hi = 0.f, lo = 0.f;
+	__device__ __forceinline__ void add(float x)
+	{
+		float s = hi + x, b = s - hi;
+		lo += (hi - (s - b)) + (x - b);
+		hi = s;
+	}
+	// (an infinite sum leaves no lo)
+	__device__ __forceinline__ double get() const { return isfinite(lo) ? double(hi) + double(lo) : double(hi); }
+};
+template <int GRP, class T, int ND>
+__global__ void __launch_bounds__(kPlaqSiteThreads, kPlaqSiteBlocks<T>)
+    k_plaquette_site(Geom g, T const *__restrict__ U, RedSlot out)
+{
+	using Gp = Group<GRP, T>;
+	using E = typename Gp::E;
+	LinkLoad<GRP, T, ND> ld{U, g.V};
+	Sum<T> acc;
+	for (int64_t s = int64_t(blockIdx.x) * kPlaqSiteThreads + threadIdx.x; s < g.V; s += int64_t(gridDim.x) * kPlaqSiteThreads)
+	{
+		Site<ND> st = site_from_eo<ND>(g, s);
+		E u[ND];
+		int32_t f[ND];
+#pragma unroll
+		for (int mu = 0; mu < ND; ++mu)
+		{
+			u[mu] = ld(mu, s);
+			f[mu] = int32_t(eo_shift1<ND>(g, st, mu, +1));
+		}
+#pragma unroll
+		for (int mu = 0; mu < ND; ++mu)
+#pragma unroll
+			for (int nu = mu + 1; nu < ND; ++nu)
+				acc.add(Gp::retr_nd(Gp::mul(u[mu], ld(nu, f[mu])), Gp::mul(u[nu], ld(mu, f[nu]))));
+	}
+	grid_sum<kPlaqSiteThreads>(acc.get(), out);
+}
+template <int GRP, class T, int ND, bool ROWS = false>
+inline void launch_plaquette(int num_sms, Geom const &g, T const *U, cudaStream_t stream, RedSlot out)
+{
+	unsigned blocks = plaquette_grid<GRP, T, ND>(num_sms, g.V);
+	if constexpr (GRP != SU3)
+		if (plaquette_by_site<GRP, T>(g.V))
+		{
+			k_plaquette_site<GRP, T, ND><<<blocks, kPlaqSiteThreads, 0, stream>>>(g, U, out);
+			MESH_LAUNCH_CHECK();
+			return;
+		}
+	if constexpr (GRP == SU3 || sizeof(T) == 8)
+		k_plaquette<GRP, T, ND, ROWS><<<blocks, kPlaqThreads, 0, stream>>>(g, U, out);
+	MESH_LAUNCH_CHECK();
 }
 
 // F[mu] += x, F[nu] -= x for the plane q (a runtime index): a chain of
@@ -2137,9 +2225,7 @@ template <int GRP, class T, int ND> struct Ops
 	static void plaquette(Field const &U, RedSlot out)
 	{
 		auto &c = *U.ctx;
-		k_plaquette<GRP, T, ND><<<plaquette_grid<T>(c.num_sms, U.geom.V), 32 * kPlanes<ND>, 0, c.stream>>>(
-		    U.geom, static_cast<T const *>(U.d), out);
-		MESH_LAUNCH_CHECK();
+		launch_plaquette<GRP, T, ND>(c.num_sms, U.geom, static_cast<T const *>(U.d), c.stream, out);
 	}
 	// the HMC trajectory's versions: SU(3) FP32 links read as rows 0, 1
 	static void hmc_plaquette(Field const &U, RedSlot out)
@@ -2147,9 +2233,7 @@ template <int GRP, class T, int ND> struct Ops
 		if constexpr (kRows<GRP, T>)
 		{
 			auto &c = *U.ctx;
-			k_plaquette<GRP, T, ND, true><<<plaquette_grid<T>(c.num_sms, U.geom.V), 32 * kPlanes<ND>, 0, c.stream>>>(
-			    U.geom, static_cast<T const *>(U.d), out);
-			MESH_LAUNCH_CHECK();
+			launch_plaquette<GRP, T, ND, true>(c.num_sms, U.geom, static_cast<T const *>(U.d), c.stream, out);
 		}
 		else
 			plaquette(U, out);

@@ -8,7 +8,7 @@
 // be created. They keep the links in their own device buffer and call this
 // function with plain pointers.
 //
-// The kernel is the one mesh_plaquette launches (k_plaquette), with the same
+// The kernel is the one mesh_plaquette launches (launch_plaquette), with the same
 // grid, so the two entry points return the same bits. Its reduction scratch
 // (one FP64 partial sum per block, the result and the last-block counter)
 // lives in the file-scope device array below instead of context memory.
@@ -89,21 +89,29 @@ void check_links(int device, void const *links)
 		throw Error(MESH_ERR_ARG, "links: the buffer belongs to another device");
 }
 
+// the grid mesh_plaquette uses on this device (a function of the lattice and the SM
+// count only); a grid beyond the scratch is refused rather than shrunk, as a different
+// grid would change the summation order
 template <int GRP, class T, int ND>
-void launch(Geom const &g, void const *links, unsigned blocks, cudaStream_t st, RedSlot slot)
+void launch(Geom const &g, void const *links, int num_sms, cudaStream_t st, RedSlot slot)
 {
-	k_plaquette<GRP, T, ND><<<blocks, 32 * kPlanes<ND>, 0, st>>>(g, static_cast<T const *>(links), slot);
+	require(plaquette_grid<GRP, T, ND>(num_sms, g.V) <= kNoAllocMaxBlocks,
+	        "mesh_plaquette_noalloc: the reduction needs more blocks than MESH_NOALLOC_MAX_BLOCKS");
+	// the last-block counter must start at zero; a finished reduction
+	// leaves it at zero, this also covers one cut short by an error
+	MESH_CUDA(cudaMemsetAsync(slot.counter, 0, sizeof(unsigned), st));
+	launch_plaquette<GRP, T, ND>(num_sms, g, static_cast<T const *>(links), st, slot);
 }
 
 template <int GRP, class T>
-void launch_nd(int nd, Geom const &g, void const *links, unsigned blocks, cudaStream_t st, RedSlot slot)
+void launch_nd(int nd, Geom const &g, void const *links, int num_sms, cudaStream_t st, RedSlot slot)
 {
 	if (nd == 2)
-		launch<GRP, T, 2>(g, links, blocks, st, slot);
+		launch<GRP, T, 2>(g, links, num_sms, st, slot);
 	else if (nd == 3)
-		launch<GRP, T, 3>(g, links, blocks, st, slot);
+		launch<GRP, T, 3>(g, links, num_sms, st, slot);
 	else
-		launch<GRP, T, 4>(g, links, blocks, st, slot);
+		launch<GRP, T, 4>(g, links, num_sms, st, slot);
 }
 
 } // namespace
@@ -135,36 +143,26 @@ extern "C" int mesh_plaquette_noalloc(int device, int group, int precision, int 
 		if (char const *why = setup(device, d))
 			throw Error(MESH_ERR_CUDA, why);
 		check_links(device, links);
-		// the grid mesh_plaquette uses on this device (a function of the volume
-		// and the SM count only); a grid beyond the scratch is refused rather
-		// than shrunk, as a different grid would change the summation order
-		unsigned blocks = precision == MESH_F32 ? plaquette_grid<float>(d.num_sms, V) : plaquette_grid<double>(d.num_sms, V);
-		require(blocks <= kNoAllocMaxBlocks,
-		        "mesh_plaquette_noalloc: the reduction needs more blocks than MESH_NOALLOC_MAX_BLOCKS");
 		auto st = static_cast<cudaStream_t>(stream);
 		RedSlot slot{d.scratch, d.scratch + kNoAllocMaxBlocks,
 		             reinterpret_cast<unsigned *>(d.scratch + kNoAllocMaxBlocks + 1)};
-		// the last-block counter must start at zero; a finished reduction
-		// leaves it at zero, this also covers one cut short by an error
-		MESH_CUDA(cudaMemsetAsync(slot.counter, 0, sizeof(unsigned), st));
 		Geom g = make_geom(nd, dims);
 		bool f32 = precision == MESH_F32;
 		switch (group)
 		{
 		case 1:
-			f32 ? launch_nd<1, float>(nd, g, links, blocks, st, slot)
-			    : launch_nd<1, double>(nd, g, links, blocks, st, slot);
+			f32 ? launch_nd<1, float>(nd, g, links, d.num_sms, st, slot)
+			    : launch_nd<1, double>(nd, g, links, d.num_sms, st, slot);
 			break;
 		case 2:
-			f32 ? launch_nd<2, float>(nd, g, links, blocks, st, slot)
-			    : launch_nd<2, double>(nd, g, links, blocks, st, slot);
+			f32 ? launch_nd<2, float>(nd, g, links, d.num_sms, st, slot)
+			    : launch_nd<2, double>(nd, g, links, d.num_sms, st, slot);
 			break;
 		default:
-			f32 ? launch_nd<3, float>(nd, g, links, blocks, st, slot)
-			    : launch_nd<3, double>(nd, g, links, blocks, st, slot);
+			f32 ? launch_nd<3, float>(nd, g, links, d.num_sms, st, slot)
+			    : launch_nd<3, double>(nd, g, links, d.num_sms, st, slot);
 			break;
 		}
-		MESH_LAUNCH_CHECK();
 		double s = 0.0;
 		MESH_CUDA(cudaMemcpyAsync(&s, slot.result, sizeof(double), cudaMemcpyDeviceToHost, st));
 		MESH_CUDA(cudaStreamSynchronize(st));
