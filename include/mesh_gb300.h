@@ -83,7 +83,9 @@ int mesh_tune_force_variant(int variant);
 /* ---- context: device + stream + reduction scratch ------------------------
  * Replaces the reference's implicit "current device, default stream"
  * (src/lattice/device.h:219-228). stream == NULL: the context creates and
- * owns a non-blocking stream. */
+ * owns a non-blocking stream. Calls that need scratch share a workspace that the
+ * context keeps until it is destroyed, at most 512 MB; what a call needs beyond
+ * that it allocates and frees. */
 int mesh_ctx_create(int device, void *stream, mesh_ctx *out);
 int mesh_ctx_destroy(mesh_ctx ctx);
 int mesh_ctx_synchronize(mesh_ctx ctx);
@@ -242,9 +244,13 @@ int mesh_reunitize(mesh_field U);
 int mesh_evolve(mesh_field U, mesh_field P, double t);
 /* P_mu -= wilsonDeriv(U, mu, beta) * delta for all mu (the momentum step
  * of runHmd, hmc.h:54-58), fused: staples, product, projection and update
- * in one kernel */
+ * in one kernel; FP64 SU(3) in two, through scratch of the size a chain's has, from
+ * the context's workspace (beyond 512 MB allocated for the call; without memory for
+ * it, and while the stream is captured, in one) */
 int mesh_momentum_step(mesh_field P, mesh_field U, double beta, double delta);
-/* runHmd (hmc.h:38-59): alternating position/momentum steps */
+/* runHmd (hmc.h:38-59): alternating position/momentum steps. A second buffer of
+ * links, and the scratch of mesh_momentum_step, come from the context's workspace;
+ * where both exceed 512 MB the steps need no second buffer */
 int mesh_run_hmd(mesh_field U, mesh_field P, double beta, const double *deltas, int n);
 /* makeDeltas (hmc.cpp:7-51): scheme "2lf", "2mn" or "4mn"; writes at most
  * capacity values and the count to *n */
@@ -255,9 +261,10 @@ int mesh_make_deltas(const char *scheme, double epsilon, int substeps, double *o
  * from counter-based device streams keyed by `seed` and the trajectory
  * number; H_old/H_new, dH and the accept decision are computed on the device
  * in FP64. The SU(3) chains of a context share the scratch of a
- * molecular-dynamics step (192 bytes a site in FP32, 2112 in FP64, of the largest
- * chain, at most 256 MB, or two slices of dimension 0 where those are more); a
- * chain made without the memory for it runs the kernels that need none. */
+ * molecular-dynamics step (in four dimensions 192 bytes a site in FP32, 2112 in FP64,
+ * of the largest chain, at most 256 MB, or two slices of dimension 0 where those are
+ * more but within 512 MB or a quarter of the links). A chain whose slices are larger,
+ * or made without the memory for it, runs the kernels that need none. */
 typedef struct mesh_hmc_record
 {
 	double plaquette; /* plaquette(U) after the accept/reject step */
@@ -366,7 +373,8 @@ int mesh_landau_theta(mesh_field U, mesh_field g, double *out);
  * landau.h:52-65); F a single-component algebra field */
 int mesh_landau_deriv(mesh_field F, mesh_field U, mesh_field g);
 /* the reference's nonlinear CG with line search (Landau::run,
- * landau.h:100-136) with the stopping threshold as an argument */
+ * landau.h:100-136) with the stopping threshold as an argument; two algebra fields
+ * and a transform from the context's workspace */
 int mesh_landau_cg(mesh_field U, mesh_field g, int max_iter, double tol, int *iters, double *theta);
 /* checkerboard overrelaxation (no reference counterpart; the legacy
  * relaxation of src/old/gauge_fixing.cpp:33-79 overrelaxed): sweeps in

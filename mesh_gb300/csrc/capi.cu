@@ -269,7 +269,7 @@ struct Workspace
 	bool own = false;
 	Workspace(Context &ctx, size_t bytes) : c(ctx)
 	{
-		if (bytes <= Context::kWorkCap && !capturing(c) && c.grow_work(bytes))
+		if (!capturing(c) && c.grow_work(bytes))
 			d = c.d_work;
 		else
 		{
@@ -299,17 +299,39 @@ Field site_field(Field const &U, int kind, void *d)
 }
 size_t site_bytes_aligned(Field const &U, int kind) { return (site_field(U, kind, nullptr).bytes + 255) / 256 * 256; }
 
-// scratch for the momentum step on U's lattice from the context's workspace. Empty
-// (the step then runs without it) while the stream is being captured, as a later
-// call may replace the memory a captured launch points to, and without memory.
-MdScratch ctx_md_scratch(Field const &U)
+// Scratch for the momentum steps of a call on U's lattice: the context's workspace, or
+// beyond its bound the call's own memory. Empty (the steps then run without it) while
+// the stream is being captured, as a later call may replace the memory a captured
+// launch points to, and without memory.
+struct CallMdScratch : MdScratch
 {
-	Context &c = *U.ctx;
-	size_t need = ops_for(U).md_scratch_bytes(U.geom, false);
-	if (need == 0 || capturing(c) || !c.grow_work(need))
-		return {};
-	return {c.d_work, c.work_bytes};
-}
+	Context &c;
+	bool own = false;
+	explicit CallMdScratch(Field const &U) : c(*U.ctx)
+	{
+		size_t need = ops_for(U).md_scratch_bytes(U.geom, false);
+		if (need == 0 || capturing(c))
+			return;
+		if (c.grow_work(need))
+			d = c.d_work;
+		else if (need <= Context::kWorkCap || cudaMallocAsync(&d, need, c.stream) != cudaSuccess)
+		{
+			cudaGetLastError();
+			d = nullptr;
+			return;
+		}
+		else
+			own = true;
+		bytes = need;
+	}
+	~CallMdScratch()
+	{
+		if (own)
+			cudaFreeAsync(d, c.stream);
+	}
+	CallMdScratch(CallMdScratch const &) = delete;
+	CallMdScratch &operator=(CallMdScratch const &) = delete;
+};
 
 void check_deltas(double const *deltas, int n)
 {
@@ -1026,7 +1048,7 @@ int mesh_momentum_step(mesh_field Ph, mesh_field Uh, double beta, double delta)
 		same_shape(U, P);
 		require(P.kind == MESH_ALGEBRA && P.nstack == U.nstack, "momenta must be an algebra field like U");
 		DeviceGuard dg(U.ctx->device);
-		ops_for(U).momentum_step(P, U, beta / (2.0 * group_nc(U.group)) * delta, nullptr, ctx_md_scratch(U));
+		ops_for(U).momentum_step(P, U, beta / (2.0 * group_nc(U.group)) * delta, nullptr, CallMdScratch(U));
 	});
 }
 
@@ -1047,11 +1069,10 @@ int mesh_run_hmd(mesh_field Uh, mesh_field Ph, double beta, double const *deltas
 		// need not hold.
 		Context &c = *U.ctx;
 		size_t need = ops.md_scratch_bytes(U.geom, false), at = (need + 255) / 256 * 256;
-		bool fuse = (U.group != 3 || U.prec == MESH_F64) && n >= 3 && !capturing(c) &&
-		            at + U.bytes <= Context::kWorkCap && c.grow_work(at + U.bytes);
+		bool fuse = (U.group != 3 || U.prec == MESH_F64) && n >= 3 && !capturing(c) && c.grow_work(at + U.bytes);
 		if (!fuse)
 		{
-			MdScratch scratch = ctx_md_scratch(U);
+			CallMdScratch scratch(U);
 			for (int i = 0; i < n; ++i)
 				if (i % 2 == 0)
 					ops.evolve(U, U, P, deltas[i], false);

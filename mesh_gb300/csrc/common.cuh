@@ -69,12 +69,14 @@ struct Context
 	// workspace of calls on plain fields (products of a momentum step, lines of
 	// Wilson loops): on this context's stream, so calls use it one after another;
 	// grown on demand, freed with the context
-	static constexpr size_t kWorkCap = size_t(512) << 20; // kept between calls at most
+	static constexpr size_t kWorkCap = size_t(512) << 20; // the most that is kept
 	void *d_work = nullptr;
 	size_t work_bytes = 0;
-	// false (and no workspace) when there is no memory
+	// false for more than is kept, and (with no workspace) when there is no memory
 	bool grow_work(size_t bytes)
 	{
+		if (bytes > kWorkCap)
+			return false;
 		if (work_bytes >= bytes)
 			return true;
 		cudaStreamSynchronize(stream);

@@ -2685,6 +2685,7 @@ template <int GRP, class T, int ND> struct Ops
 	// unitary: md_plaquettes.cuh) -------------------------------------------------
 	static constexpr bool kProducts = GRP == SU3 && sizeof(T) == 8;
 	static constexpr bool kPlaquettes = kRows<GRP, T>;
+	static constexpr size_t kLinkBytes = sizeof(T) * ND * Gp::NR; // links of a site
 	// bytes of scratch a site; rows: links known to be special unitary
 	static size_t md_site_bytes(bool rows)
 	{
@@ -2698,7 +2699,7 @@ template <int GRP, class T, int ND> struct Ops
 		if (kPlaquettes && !LinkLoadSU3R32::fits(g.V))
 			site = 0; // 32-bit offsets
 		if (site)
-			md_ring(g, site, &bytes);
+			md_ring(g, site, kLinkBytes * size_t(g.V), &bytes);
 		return bytes;
 	}
 	// walks the lattice: first(x0, n, t0) fills the ring, second(x0, n) uses it
@@ -2726,7 +2727,7 @@ template <int GRP, class T, int ND> struct Ops
 		size_t bytes = md_scratch_bytes(g, rows);
 		if (!bytes || scratch.bytes < bytes)
 			return false;
-		MdRing ring = md_ring(g, md_site_bytes(rows), &bytes);
+		MdRing ring = md_ring(g, md_site_bytes(rows), kLinkBytes * size_t(g.V), &bytes);
 		// a sum over several launches: after them, from P
 		RedSlot slot = kin && ring.whole ? *kin : RedSlot{};
 		if constexpr (kProducts)

@@ -23,12 +23,15 @@
 //
 // Scratch: the products of the whole lattice when they fit kMdScratchCap, else
 // a ring of R slices of dimension 0 (a slice's forces read the products of its
-// own and of the preceding slice), walked in slabs of R - 1 slices.
+// own and of the preceding slice), walked in slabs of R - 1 slices: two slices
+// at least, where they fit kMdScratchMax or a quarter of the links. A lattice
+// with larger slices steps without scratch, by the kernels of kernels.cuh.
 #pragma once
 
 namespace meshgb {
 
 constexpr size_t kMdScratchCap = size_t(256) << 20;
+constexpr size_t kMdScratchMax = size_t(512) << 20;
 
 // Slices of dimension 0 whose products are held, S sites each
 struct MdRing
@@ -150,20 +153,18 @@ __global__ void __launch_bounds__(32 * ND)
 		grid_sum<32 * ND>(acc, kin);
 }
 
-// the ring of a lattice within the cap (site_bytes held for a site), and its bytes
-inline MdRing md_ring(Geom const &g, size_t site_bytes, size_t *bytes)
+// the ring of a lattice (site_bytes held for a site, link_bytes of links) and its
+// bytes; none (R = 0) where two slices are too large
+inline MdRing md_ring(Geom const &g, size_t site_bytes, size_t link_bytes, size_t *bytes)
 {
 	MdRing r{};
 	r.S = g.V / g.L[0];
 	size_t slice = size_t(r.S) * site_bytes;
 	int64_t fit = int64_t(kMdScratchCap / slice);
-	r.whole = fit >= g.L[0];
-	r.R = r.whole ? g.L[0] : int(fit < 2 ? 2 : fit);
-	if (!r.whole && r.R >= g.L[0])
-	{
-		r.whole = 1; // two slices are the lattice
-		r.R = g.L[0];
-	}
+	if (fit < 2)
+		fit = 2 * slice <= kMdScratchMax || 2 * slice <= link_bytes / 4 ? 2 : 0;
+	r.R = int(fit < g.L[0] ? fit : g.L[0]);
+	r.whole = r.R == g.L[0];
 	r.V = r.R * r.S;
 	*bytes = slice * size_t(r.R);
 	return r;
