@@ -883,10 +883,10 @@ int mesh_batch_create(mesh_ctx ctxh, int group, int precision, int nrep, int32_t
 			totU += align(size_t(kBND) * size_t(V) * nr * rb);
 			totP += align(size_t(kBND) * size_t(V) * na * rb);
 		}
-		MESH_CUDA(cudaMalloc(&h->bufU, totU));
-		MESH_CUDA(cudaMalloc(&h->bufUnew, totU));
-		MESH_CUDA(cudaMalloc(&h->bufUt, totU));
-		MESH_CUDA(cudaMalloc(&h->bufP, totP));
+		h->bufU = c.alloc(totU);
+		h->bufUnew = c.alloc(totU);
+		h->bufUt = c.alloc(totU);
+		h->bufP = c.alloc(totP);
 		for (int r = 0; r < nrep; ++r)
 		{
 			h->reps[r].U = static_cast<char *>(h->bufU) + offU[r];

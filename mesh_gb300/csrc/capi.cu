@@ -125,7 +125,7 @@ void create_field(Context &c, int kind, int group, int prec, int nd, int32_t con
 	f.real_bytes = prec == MESH_F32 ? 4 : 8;
 	f.bytes = size_t(nstack) * size_t(V) * size_t(f.nr) * f.real_bytes;
 	DeviceGuard dg(c.device);
-	MESH_CUDA(cudaMalloc(&f.d, f.bytes));
+	f.d = c.alloc(f.bytes);
 	++c.refs;
 }
 
@@ -273,7 +273,7 @@ struct Workspace
 			d = c.d_work;
 		else
 		{
-			MESH_CUDA(cudaMallocAsync(&d, bytes, c.stream));
+			d = c.alloc(bytes, true);
 			own = true;
 		}
 	}

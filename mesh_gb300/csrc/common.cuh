@@ -68,7 +68,7 @@ struct Context
 
 	// workspace of calls on plain fields (products of a momentum step, lines of
 	// Wilson loops): on this context's stream, so calls use it one after another;
-	// grown on demand, freed with the context
+	// grown on demand, freed with the context or when an allocation wants the memory
 	static constexpr size_t kWorkCap = size_t(512) << 20; // the most that is kept
 	void *d_work = nullptr;
 	size_t work_bytes = 0;
@@ -100,13 +100,49 @@ struct Context
 	std::shared_ptr<void> md_shared;
 	size_t md_shared_bytes = 0;
 
+	// frees what is kept only to be used again; false when there is nothing, or while
+	// the stream is captured
+	bool give_back()
+	{
+		cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+		bool shared = md_shared && md_shared.use_count() == 1;
+		if ((!d_work && !shared) || cudaStreamIsCapturing(stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone)
+			return false;
+		cudaStreamSynchronize(stream);
+		cudaFree(d_work);
+		d_work = nullptr;
+		work_bytes = 0;
+		if (shared)
+		{
+			md_shared.reset();
+			md_shared_bytes = 0;
+		}
+		return true;
+	}
+	// device memory that outlives the call (async: of the stream's pool); one that the
+	// kept workspaces leave no room for takes them back
+	void *alloc(size_t bytes, bool async = false)
+	{
+		void *p = nullptr;
+		auto get = [&] { return async ? cudaMallocAsync(&p, bytes, stream) : cudaMalloc(&p, bytes); };
+		cudaError_t e = get();
+		if (e == cudaErrorMemoryAllocation && give_back())
+			e = get();
+		cudaGetLastError(); // not left for the next launch's check
+		MESH_CUDA(e);
+		return p;
+	}
+
 	void *stage(size_t bytes)
 	{
 		if (bytes > stage_bytes)
 		{
-			if (d_stage)
-				MESH_CUDA(cudaFreeAsync(d_stage, stream));
-			MESH_CUDA(cudaMallocAsync(&d_stage, bytes, stream));
+			void *old = d_stage;
+			d_stage = nullptr;
+			stage_bytes = 0;
+			if (old)
+				MESH_CUDA(cudaFreeAsync(old, stream));
+			d_stage = alloc(bytes, true);
 			stage_bytes = bytes;
 		}
 		return d_stage;

@@ -193,10 +193,11 @@ int mesh_landau_fa_create(mesh_field Uh, mesh_landau_fa_s **out)
 		h->nf = (na + 1) / 2;
 		int64_t V = U.geom.V;
 		DeviceGuard dg(U.ctx->device);
-		MESH_CUDA(cudaMalloc(&h->A, sizeof(double) * size_t(U.nd) * na * V));
-		MESH_CUDA(cudaMalloc(&h->buf, sizeof(float2) * size_t(h->nf) * V));
-		MESH_CUDA(cudaMalloc(&h->buf_old, sizeof(float2) * size_t(h->nf) * V));
-		MESH_CUDA(cudaMalloc(&h->g_trial, sizeof(double) * size_t(group_nr(U.group)) * V));
+		auto &c = *U.ctx;
+		h->A = static_cast<double *>(c.alloc(sizeof(double) * size_t(U.nd) * na * V));
+		h->buf = static_cast<float2 *>(c.alloc(sizeof(float2) * size_t(h->nf) * V));
+		h->buf_old = static_cast<float2 *>(c.alloc(sizeof(float2) * size_t(h->nf) * V));
+		h->g_trial = static_cast<double *>(c.alloc(sizeof(double) * size_t(group_nr(U.group)) * V));
 		MESH_CUDA(cudaMalloc(&h->red, sizeof(double) * 2 * kMaxRedBlocks));
 		MESH_CUDA(cudaMalloc(&h->res, sizeof(double) * 2));
 		MESH_CUDA(cudaMalloc(&h->cnt, sizeof(unsigned) * 2));
@@ -558,8 +559,7 @@ extern "C" int mesh_lattice_fft(mesh_ctx ctx, int nd, int32_t const *dims, int n
 		Context &c = ctx->c;
 		DeviceGuard dg(c.device);
 		size_t bytes = sizeof(float2) * size_t(nf) * size_t(V);
-		float2 *d = nullptr;
-		MESH_CUDA(cudaMallocAsync(&d, bytes, c.stream));
+		auto *d = static_cast<float2 *>(c.alloc(bytes, true));
 		MESH_CUDA(cudaMemcpyAsync(d, data, bytes, cudaMemcpyHostToDevice, c.stream));
 		if (sign < 0)
 			fft::fft_nd<-1>(d, nd, dims, nf, c.num_sms, c.stream);

@@ -87,3 +87,36 @@ def test_run_hmd_without_the_second_buffer(own, g, p, dims):
     mg.evolve(W, Q, d[2])
     assert distance(P, Q) < (1e-14 if p == 2 else 1e-6)
     assert mg.plaquette(U) == pytest.approx(mg.plaquette(W), abs=1e-13 if p == 2 else 1e-8)
+
+
+@pytest.mark.parametrize("kept", ["workspace", "chains"])
+def test_kept_memory_is_given_back_to_an_allocation(own, kept):
+    """with 200 MB free, a field of 302 MB finds the 256 MB or more that the context keeps"""
+    grid = mg.Grid([64, 16, 16, 16])
+    if kept == "workspace":
+        U, P = mg.GaugeField(own, 3, 2, grid).random(1), mg.Momenta(own, 3, 2, grid).random(2)
+        mg.momentum_step(P, U, 5.7, 0.1)
+        own.synchronize()
+        U.close()
+        P.close()
+    else:
+        mg.Hmc(own, 3, 2, grid, seed=1).close()
+    torch.cuda.empty_cache()
+    hog = torch.empty(free_bytes() - 200 * MB, dtype=torch.uint8, device="cuda")
+    try:
+        assert free_bytes() < 220 * MB
+        f = mg.GaugeField(own, 3, 1, mg.Grid([32] * 4))
+        f.set_unit()
+        assert mg.plaquette(f) == 1.0
+        f.close()
+    finally:
+        del hog
+        torch.cuda.empty_cache()
+
+
+def test_refused_allocation_leaves_the_context_usable(own):
+    """a field larger than the device (1.2e9 sites of FP64 SU(3): 702 GB) is refused, and
+    the next call does not find the error"""
+    with pytest.raises(mg.MeshError, match="out of memory"):
+        mg.GaugeField(own, 3, 2, mg.Grid([186] * 4))
+    assert mg.plaquette(mg.GaugeField(own, 3, 2, mg.Grid([4] * 4)).set_unit()) == 1.0
