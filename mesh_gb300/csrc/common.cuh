@@ -79,18 +79,23 @@ struct Context
 			return false;
 		if (work_bytes >= bytes)
 			return true;
+		// the calls that come here wait for nothing and allocate nothing else: a capture of
+		// another stream, on this thread or another, must not be invalidated here
+		cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+		cudaThreadExchangeStreamCaptureMode(&mode);
 		cudaStreamSynchronize(stream);
 		cudaFree(d_work);
 		d_work = nullptr;
 		work_bytes = 0;
-		if (cudaMalloc(&d_work, bytes) != cudaSuccess)
+		if (cudaMalloc(&d_work, bytes) == cudaSuccess)
+			work_bytes = bytes;
+		else
 		{
 			cudaGetLastError();
 			d_work = nullptr;
-			return false;
 		}
-		work_bytes = bytes;
-		return true;
+		cudaThreadExchangeStreamCaptureMode(&mode);
+		return work_bytes > 0;
 	}
 
 	// scratch of the chains' molecular-dynamics steps, one for all chains of the

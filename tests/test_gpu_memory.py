@@ -120,3 +120,27 @@ def test_refused_allocation_leaves_the_context_usable(own):
     with pytest.raises(mg.MeshError, match="out of memory"):
         mg.GaugeField(own, 3, 2, mg.Grid([186] * 4))
     assert mg.plaquette(mg.GaugeField(own, 3, 2, mg.Grid([4] * 4)).set_unit()) == 1.0
+
+
+def test_workspace_grows_beside_a_capture(own):
+    """FP64 SU(3) steps that need a (larger) workspace, on the context's stream, while
+    the thread captures another stream: the capture stays valid, the momenta are those
+    of a step without one"""
+    x = torch.zeros(64, device="cuda")
+    fields = []
+    for dims in ([4, 4, 4, 8], [8, 8, 8, 8]):
+        grid = mg.Grid(dims)
+        U, P = mg.GaugeField(own, 3, 2, grid).random(1), mg.Momenta(own, 3, 2, grid).random(2)
+        fields.append((U, P, mg.Momenta(own, 3, 2, grid).copy_from(P)))
+    own.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        x += 1
+        for U, P, _ in fields:
+            mg.momentum_step(P, U, 5.7, 0.3)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert float(x[0]) == 1.0
+    for U, P, Q in fields:
+        mg.momentum_step(Q, U, 5.7, 0.3)
+        assert distance(P, Q) < 1e-15
