@@ -3013,7 +3013,11 @@ template <int GRP, class T, int ND> struct Ops
 		int v = tuned_variant(key);
 		if (v >= 0)
 			return v;
-		int dflt = force_variant_valid(U.geom, 3) ? 3 : 0;
+		// where nothing is timed. FP64 SU(3) steps by stored products where it can, and so is
+		// never timed before a capture of a plain field's step: in even/odd order, which was
+		// the fastest or within 4% of it wherever they were timed (8^4 96 us, 371 by tiles;
+		// 12^3x24 459 and 734, 16^4 640 and 735)
+		int dflt = !kProducts && force_variant_valid(U.geom, 3) ? 3 : 0;
 		cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
 		cudaStreamIsCapturing(U.ctx->stream, &cs);
 		if (cs != cudaStreamCaptureStatusNone || !autotune_enabled())
