@@ -76,7 +76,8 @@ int mesh_version(void);
  * environment disables it (default variants). */
 size_t mesh_tune_report(char *buf, size_t cap);
 /* Forces launch variant `variant` of the fused momentum-step kernel for all
- * later calls where it is valid for the lattice (-1 restores autotuning).
+ * later calls where it is valid for the lattice (-1 restores autotuning; 59: the
+ * SU(3) steps through scratch, where there is scratch).
  * For testing every variant against the oracle. */
 int mesh_tune_force_variant(int variant);
 

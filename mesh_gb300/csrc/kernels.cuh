@@ -2857,6 +2857,10 @@ template <int GRP, class T, int ND> struct Ops
 	// stream is capturing
 	static constexpr int kSeparate = 1000; // the two steps as separate kernels were faster
 	static constexpr int kStored = 1001;   // the step from stored plaquettes was faster
+	// pins the SU(3) steps through scratch (stored products, stored plaquettes)
+	static constexpr int kPinScratch = 59;
+	static_assert(kPinScratch >= kForceVariants);
+	static bool products_allowed() { return kProducts && (force_override() < 0 || force_override() == kPinScratch); }
 	static bool stored_applies(Geom const &g, MdScratch const &scratch)
 	{
 		return kPlaquettes && scratch.bytes >= md_scratch_bytes(g, true) && md_scratch_bytes(g, true) > 0;
@@ -2867,20 +2871,23 @@ template <int GRP, class T, int ND> struct Ops
 		int ov = force_override();
 		if (ov >= kMdFirst && ov <= kMdLast && force_variant_valid(Uin.geom, ov))
 			return ov;
+		if (ov == kPinScratch && stored)
+			return kStored;
 		if (ov >= 0 && ov < kMdFirst)
 			return kSeparate; // a thread-per-link variant pinned: no fusion
 		std::string key = "md_step/group" + std::to_string(GRP) + "/" + (sizeof(T) == 4 ? "f32" : "f64") + "/";
 		for (int i = 0; i < ND; ++i)
 			key += (i ? "x" : "") + std::to_string(Uin.dims[i]);
-		// where nothing is timed, and for a chain without the scratch that the
-		// lattice was tuned with
+		if (kPlaquettes && !stored)
+			key += "/no scratch"; // times fewer steps than the lattice's other chains
+		// where nothing is timed
 		int dflt = stored ? kStored : kSeparate;
 		for (int cand = kMdFirst; cand <= kMdLast && dflt == kSeparate; ++cand)
 			if (force_variant_valid(Uin.geom, cand))
 				dflt = cand;
 		int v = tuned_variant(key);
 		if (v >= 0)
-			return v == kStored && !stored ? dflt : v;
+			return v;
 		cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
 		cudaStreamIsCapturing(Uin.ctx->stream, &cs);
 		if (cs != cudaStreamCaptureStatusNone || !autotune_enabled())
@@ -2971,7 +2978,7 @@ template <int GRP, class T, int ND> struct Ops
 	static bool hmc_md_step(Field &P, Field const &Uin, Field &Uout, double coef, double tu, bool reunit,
 	                        RedSlot *kin, MdScratch const &scratch, bool row2)
 	{
-		if (kProducts && force_override() < 0 && scratch_step(P, Uin, &Uout, coef, tu, reunit, kin, scratch, true))
+		if (products_allowed() && scratch_step(P, Uin, &Uout, coef, tu, reunit, kin, scratch, true))
 			return true;
 		if (!md_supported(Uin.geom) && !stored_applies(Uin.geom, scratch))
 			return false;
@@ -2987,7 +2994,7 @@ template <int GRP, class T, int ND> struct Ops
 	// step from stored products has none
 	static void hmc_tune_md(Field &P, Field const &Uin, Field &Uout, MdScratch const &scratch)
 	{
-		if (kProducts && force_override() < 0 && scratch.bytes >= md_scratch_bytes(Uin.geom, true))
+		if (products_allowed() && scratch.bytes >= md_scratch_bytes(Uin.geom, true))
 			return;
 		choose_force(P, Uin, true);
 		if (md_supported(Uin.geom) || stored_applies(Uin.geom, scratch))
@@ -3057,14 +3064,14 @@ template <int GRP, class T, int ND> struct Ops
 	}
 	static void momentum_step(Field &P, Field const &U, double coef, RedSlot *kin, MdScratch const &scratch)
 	{
-		if (kProducts && force_override() < 0 && scratch_step(P, U, nullptr, coef, 0.0, false, kin, scratch, false))
+		if (products_allowed() && scratch_step(P, U, nullptr, coef, 0.0, false, kin, scratch, false))
 			return;
 		int v = choose_force(P, U);
 		launch_force(v, P, U, T(coef), kin ? *kin : RedSlot{});
 	}
 	static void hmc_momentum_step(Field &P, Field const &U, double coef, RedSlot *kin, MdScratch const &scratch)
 	{
-		if (kProducts && force_override() < 0 && scratch_step(P, U, nullptr, coef, 0.0, false, kin, scratch, true))
+		if (products_allowed() && scratch_step(P, U, nullptr, coef, 0.0, false, kin, scratch, true))
 			return;
 		int v = choose_force(P, U, true);
 		launch_force(v, P, U, T(coef), kin ? *kin : RedSlot{}, true);
