@@ -1520,12 +1520,29 @@ static double landau_line_search(Field const &U, Field const &g, Field const &Fd
 		if (eps < 1e-10)
 			return 0.0;
 	}
+	// the trial at 0.8 eps is not needed where the one at 1.2 eps wins: both are made
+	// before the wait only where a trial costs no more than twice a wait (about 20 us),
+	// links of 32 MB in FP64 and 128 MB in FP32. A search won by 1.2 eps with both made
+	// and with one: SU(2) FP64 32^4 (134 MB) 1073 and 782 us, SU(3) FP64 16^4 (38 MB) 440
+	// and 326; one that needs both, made one after the other: 552 -> 564 there
+	bool both = U.bytes <= size_t(U.prec == MESH_F64 ? 32 : 128) << 20;
 	stepped(eps * 1.2, SLOT_TMP);
-	stepped(eps * 0.8, SLOT_TMP2);
-	read_slots(c, y);
-	double y2 = y[0] * norm_fac, y3 = y[1] * norm_fac;
+	if (both)
+	{
+		stepped(eps * 0.8, SLOT_TMP2);
+		read_slots(c, y);
+	}
+	else
+		y[0] = read_slot(c, SLOT_TMP);
+	double y2 = y[0] * norm_fac;
 	if (y2 > y1)
 		return 1.2 * eps;
+	if (!both)
+	{
+		stepped(eps * 0.8, SLOT_TMP2);
+		y[1] = read_slot(c, SLOT_TMP2);
+	}
+	double y3 = y[1] * norm_fac;
 	double x1 = eps, x2 = 1.2 * eps, x3 = 0.8 * eps;
 	return 0.5 * ((x2 * x2 - x3 * x3) * y1 - (x1 * x1 - x3 * x3) * y2 + (x1 * x1 - x2 * x2) * y3) /
 	       ((x2 - x3) * y1 - (x1 - x3) * y2 + (x1 - x2) * y3);

@@ -146,3 +146,38 @@ def test_chain_without_scratch(dims, lines):
     assert rel(*out) < 2e-5
     small.close()
     c.close()
+
+
+@pytest.mark.parametrize("eps", [3e3, 4e5, 1.5e6, 1e7])
+@pytest.mark.parametrize("dims", [[14, 14, 14, 16], [16, 16, 16, 16]], ids=lambda d: "x".join(map(str, d)))
+def test_line_search_trials(ctx, oracle, dims, eps):
+    """FP64 SU(3) links of 25 and 38 MB: both trials read together, and one after the
+    other; steps that grow and steps that overshoot. The step is a ratio of differences of
+    functionals that agree in some digits: 1e-6"""
+    U64, g64 = oracle.random_gauge(3, 2, dims, 4), oracle.random_transform(3, 2, dims, 5)
+    L = mg.Landau(mg.GaugeField(ctx, 3, 2, mg.Grid(dims)).import_(U64))
+    L.g.import_(g64)
+    F = L.deriv()
+    got = L.line_search(F, eps)
+    assert got == pytest.approx(oracle.landau_line_search(3, 2, dims, U64, g64, F.export(), eps), rel=1e-6)
+
+
+def test_line_search_makes_no_trial_in_vain(ctx):
+    """SU(2) FP64 32^4: a search that the longer trial wins, against one on the same
+    fields that needs the shorter one too (four trials for three): at most 0.85 of its time"""
+    U = mg.GaugeField(ctx, 2, 2, mg.Grid([32] * 4)).random(3)
+    L = mg.Landau(U)
+    F = L.deriv()
+
+    def search(eps):
+        best = 1e9
+        for _ in range(5):
+            t = time.perf_counter()
+            for _ in range(3):
+                s = L.line_search(F, eps)
+            best = min(best, time.perf_counter() - t)
+        return best, s
+
+    (t1, s1), (t2, s2) = search(1.0), search(1e7)
+    assert s1 == 1.2 and s2 > 1.3e7  # neither was halved
+    assert t1 <= 0.85 * t2
