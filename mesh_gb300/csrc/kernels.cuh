@@ -2719,13 +2719,13 @@ template <int GRP, class T, int ND> struct Ops
 			second(x0, n);
 		}
 	}
-	// false (nothing launched) without scratch or with a pinned launch variant
+	// false (nothing launched) without scratch
 	static bool scratch_step(Field &P, Field const &U, Field *Uout, double coef, double tu, bool reunit, RedSlot *kin,
 	                         MdScratch const &scratch, bool rows, bool row2 = true)
 	{
 		Geom const &g = U.geom;
 		size_t bytes = md_scratch_bytes(g, rows);
-		if (!bytes || scratch.bytes < bytes)
+		if (!bytes || scratch.bytes < bytes || (kPlaquettes && !Uout))
 			return false;
 		MdRing ring = md_ring(g, md_site_bytes(rows), kLinkBytes * size_t(g.V), &bytes);
 		// a sum over several launches: after them, from P
@@ -2735,9 +2735,9 @@ template <int GRP, class T, int ND> struct Ops
 		else if constexpr (kPlaquettes)
 		{
 			if (ring.whole)
-				plaquettes_step<true>(P, U, Uout, coef, tu, reunit, slot, ring, scratch, row2);
+				plaquettes_step<true>(P, U, *Uout, coef, tu, reunit, slot, ring, scratch, row2);
 			else
-				plaquettes_step<false>(P, U, Uout, coef, tu, reunit, slot, ring, scratch, row2);
+				plaquettes_step<false>(P, U, *Uout, coef, tu, reunit, slot, ring, scratch, row2);
 		}
 		if (kin && !ring.whole)
 			norm2(P, *kin);
@@ -2778,7 +2778,7 @@ template <int GRP, class T, int ND> struct Ops
 		}
 	}
 	template <bool WHOLE>
-	static void plaquettes_step(Field &P, Field const &U, Field *Uout, double coef, double tu, bool reunit,
+	static void plaquettes_step(Field &P, Field const &U, Field &Uout, double coef, double tu, bool reunit,
 	                            RedSlot const &kin, MdRing const &ring, MdScratch const &scratch, bool row2)
 	{
 		if constexpr (kPlaquettes)
@@ -2787,7 +2787,7 @@ template <int GRP, class T, int ND> struct Ops
 			Geom const &g = U.geom;
 			LinkLoadSU3R32 ld{static_cast<float4 const *>(U.d), uint32_t(g.V), uint32_t(g.V / 2 * 9)};
 			AlgR32 A{static_cast<float4 *>(scratch.d), uint32_t(ring.V)};
-			T *p = static_cast<T *>(P.d), *uo = Uout ? static_cast<T *>(Uout->d) : nullptr;
+			T *p = static_cast<T *>(P.d), *uo = static_cast<T *>(Uout.d);
 			md_slabs(
 			    g, ring,
 			    [&](int x0, int n, int t0) {
@@ -2797,7 +2797,7 @@ template <int GRP, class T, int ND> struct Ops
 				    MESH_LAUNCH_CHECK();
 			    },
 			    [&](int x0, int n) {
-				    auto k = Uout ? k_md_transport<ND, true, WHOLE> : k_md_transport<ND, false, WHOLE>;
+				    auto k = k_md_transport<ND, WHOLE>;
 				    constexpr int nt = 32 * ND;
 				    k<<<slab_grid(c, k, nt, ring, n), nt, 0, c.stream>>>(g, ring, x0, n, ld, A, p, T(coef), kin, uo, T(tu),
 				                                                        reunit ? 1 : 0, row2 ? 1 : 0);

@@ -6,15 +6,15 @@
 // loop of link (y + nu, mu) that starts with it is h^+ P^+ h, whose projection is
 // -h^+ A h; likewise +h^+ A h with h = U_mu(y) for link (y + mu, nu).
 //   k_md_plaquettes: A of every plane, one warp per plane for 32 sites;
-//   k_md_transport:  P_mu -= coef sum_nu +-(A(x) - h^+ A(x-nu) h) and with FUSE the
-//                    link update, one warp per direction for 32 sites.
-// About 5100 FP32 lane operations a site (6 x 316 and 4 x 730 with the index
-// arithmetic) against 6800 of the thread-per-site kernel, whose lower staples take
-// two products each, and a sixth of the chain of dependent loads a thread: any
-// extents, no tiles. The price is A (192 bytes a site written, read by the site
-// and its neighbours): 1.2 GB of DRAM traffic for a step of 32^4 where the
-// thread-per-site kernel has 0.74. The plaquettes are bound by issue (68% of the
-// slots), the transport by load latency at 24 warps per SM and 60% of HBM.
+//   k_md_transport:  P_mu -= coef sum_nu +-(A(x) - h^+ A(x-nu) h) and the link
+//                    update, one warp per direction for 32 sites.
+// 2811 and 4014 instructions a site, about what the thread-per-site kernel takes
+// (6584), whose lower staples take two products each; but a sixth of the chain of
+// dependent loads a thread, twice the warps, and any extents, no tiles. The price is
+// A (192 bytes a site written, read by the site and its neighbours): 1.2 GB of DRAM
+// traffic for a step of 32^4 where the thread-per-site kernel has 0.74. The
+// plaquettes are bound by issue (68% of the slots), the transport by load latency at
+// 24 warps per SM (61% of the slots, 4.9 TB/s of DRAM).
 // One step with the link update, SU(3) FP32 on a GB300, before and after:
 // 12x20x14x30 59.5 -> 32.9 us, 24^4 115 -> 98, 32^4 328 -> 286 (117 + 173), 8^4
 // 13.1 -> 9.0. Measured and not kept: packed FP32x2 products (the same time),
@@ -161,10 +161,10 @@ __global__ void __launch_bounds__(32 * kPlanes<ND>, ND == 4 ? 4 : 8)
 	}
 }
 
-// momentum step (and with FUSE the link update) of the slices [x0, x0 + n);
+// momentum step and link update of the slices [x0, x0 + n);
 // row2: the new links' third rows are written (the trajectory reads rows 0 and 1
 // of the links between its first and last step)
-template <int ND, bool FUSE, bool WHOLE>
+template <int ND, bool WHOLE>
 __global__ void __launch_bounds__(32 * ND, ND == 4 ? 6 : 8)
     k_md_transport(Geom g, MdRing ring, int x0, int n, LinkLoadSU3R32 ld, AlgR32 A, float *__restrict__ P, float coef,
                    RedSlot kin, float *__restrict__ Uout, float tu, int reunit, int row2)
@@ -217,26 +217,23 @@ __global__ void __launch_bounds__(32 * ND, ND == 4 ? 6 : 8)
 		Pv.template store<CACHE_STREAM>(s, p);
 		if (kin.result)
 			acc += double(Gp::kin(p));
-		if constexpr (FUSE)
+		E u = ld.rows(mu, s);
+		Gp::complete_row2(u);
+		E r = su3_rows01(Gp::exp_packed_rows01(p, tu), u);
+		if (row2)
 		{
-			E u = ld.rows(mu, s);
-			Gp::complete_row2(u);
-			E r = su3_rows01(Gp::exp_packed_rows01(p, tu), u);
-			if (row2)
-			{
-				Gp::complete_row2(r);
-				if (reunit)
-					r = Gp::reunit_fast(r);
-				comp<float, Gp::NR>(Uout, g.V, mu).store(s, r.v);
-			}
-			else
-			{
-				unitary_rows01(r);
-				float4 *U4 = reinterpret_cast<float4 *>(Uout) + (uint32_t(mu) * ld.Vmu + uint32_t(s));
+			Gp::complete_row2(r);
+			if (reunit)
+				r = Gp::reunit_fast(r);
+			comp<float, Gp::NR>(Uout, g.V, mu).store(s, r.v);
+		}
+		else
+		{
+			unitary_rows01(r);
+			float4 *U4 = reinterpret_cast<float4 *>(Uout) + (uint32_t(mu) * ld.Vmu + uint32_t(s));
 #pragma unroll
-				for (int c = 0; c < 3; ++c)
-					U4[uint32_t(c) * ld.V] = make_float4(r.v[4 * c], r.v[4 * c + 1], r.v[4 * c + 2], r.v[4 * c + 3]);
-			}
+			for (int c = 0; c < 3; ++c)
+				U4[uint32_t(c) * ld.V] = make_float4(r.v[4 * c], r.v[4 * c + 1], r.v[4 * c + 2], r.v[4 * c + 3]);
 		}
 	}
 	if (kin.result) // uniform over the grid
