@@ -83,8 +83,11 @@ struct Context
 		// another stream, on this thread or another, must not be invalidated here
 		cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
 		cudaThreadExchangeStreamCaptureMode(&mode);
-		cudaStreamSynchronize(stream);
-		cudaFree(d_work);
+		if (d_work)
+		{
+			cudaStreamSynchronize(stream);
+			cudaFree(d_work);
+		}
 		d_work = nullptr;
 		work_bytes = 0;
 		if (cudaMalloc(&d_work, bytes) == cudaSuccess)

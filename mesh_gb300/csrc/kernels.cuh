@@ -1519,7 +1519,7 @@ __global__ void __launch_bounds__(kBlock) k_spatial_lines(Geom g, int r, T const
 // spatial lines of r links, Tl: the temporal lines. Tiles of 32 sites, one warp per
 // mu: S_mu(x) stays in registers for the chunk, S_mu(x + t 3) comes from the same
 // x3 lines for every t and T_t(x) serves the three warps, both mostly from L1. What
-// bounds it is L2 to L1 (about 9 TB/s): a launch for each (r, t) read ten links a
+// bounds it is L2 to L1 (8.6 TB/s): a launch for each (r, t) read ten links a
 // site from L2, here it is a good half.
 // 24^4 SU(3) FP32 on a GB300, t = 1 .. 12 of one r: 379 us in a launch each, 240
 // here. Measured and not kept: chunks of 8 and 12 (264, 305 us), six or more blocks
