@@ -886,8 +886,8 @@ template <int ND, int NA, class T> __device__ __forceinline__ void add_dir(T (&F
 // index arithmetic, not the arithmetic of the staples, set the instruction count.
 // FINE: the kinetic norm is summed link by link in FP64, as the kernels with a thread
 // per link and H_old sum it (in the field precision, four links to an FP64 add, dH of
-// unchanged FP32 momenta was off by up to 7e-9 of H), and the link update's product
-// rounds once at the size of the link (as it came out of mul, the links of FP32 U(1)
+// unchanged FP32 momenta was off by up to 7e-9 of H), and the link update's product in
+// FP32 rounds once at the size of the link (as it came out of mul, the links of U(1)
 // and SU(2) were 9% and 5% further from FP64's after ten steps than those of the
 // separate link update; now they are as close and 24% closer). The batched replicas' kernel,
 // which spills registers, does without.
@@ -971,7 +971,7 @@ __device__ __forceinline__ double site_md_small(Geom const &g, Site<ND> const &s
 		if constexpr (FUSE)
 		{
 			E x = Gp::exp_alg(p, tu), r;
-			if constexpr (FINE)
+			if constexpr (FINE && sizeof(T) == 4)
 				r = Gp::mul_near1(x, u[mu]);
 			else
 				r = Gp::mul(x, u[mu]);
